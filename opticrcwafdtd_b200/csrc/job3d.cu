@@ -121,13 +121,57 @@ int Job3D<R>::encode_tmap3(CUtensorMap* m, CUtensorMapDataType t, const void* ba
     return ORF_OK;
 }
 
+// Segment lengths of a 3D run.  A CTA marches its segment plane by plane, a
+// serial chain: 5 us + 0.92 us a plane (CPML: 3.6 + 3.2) while the SM has little
+// else to do; a full SM spends 0.48 us (CPML 1.09) on a plane, and a segment
+// costs about five planes' worth of start.  One launch then takes about the
+// longest segment's chain plus the work shared by the SMs: short segments win
+// while the grid leaves SMs idle, long ones once it fills them.  Both lengths
+// are chosen to minimise that estimate, within kSeg3 (the constants fitted to
+// 120 timed steps of ten grids and twelve pairs of lengths on a B200, rms
+// error 15 %; the choice within 13 % of the best of the twelve on each).
+// Per step, against segments of up to kSeg3 planes: 22 x 22 x 171 periodic FP32
+// 64 -> 13 us, 201 x 93 x 77 with CPML on all sides 239 -> 85 us, 200 x 160 x
+// 141 FP64 244 -> 202 us; 320 x 320 x 200 and larger keep the long segments
+// (with shorter ones 379 -> 402 us).
+namespace {
+struct SegPlan {
+    int in, pml;   // planes of a segment at most, away from and at the z slabs
+};
+SegPlan seg_lengths(int cols_in, int cols_pml, const std::vector<std::pair<int, bool>>& zones) {
+    constexpr double kSm = 148.0, kStart = 5.1;
+    constexpr double kFixed[2] = {5.0, 3.65}, kAlone[2] = {0.92, 3.24}, kShared[2] = {0.475, 1.09};   // in, pml
+    static const int kLen[] = {60, 40, 30, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2};
+    SegPlan best{kSeg3, kSeg3};
+    double best_t = -1.0;
+    for (int li : kLen)
+        for (int lp : kLen) {
+            double chain = 0.0, work = 0.0;
+            for (auto [planes, pml] : zones) {
+                const int c = (planes + (pml ? lp : li) - 1) / (pml ? lp : li);
+                const double len = (double)planes / c;
+                const int nin = pml ? 0 : cols_in, npml = cols_in + cols_pml - nin;
+                if (nin) chain = std::max(chain, kFixed[0] + len * kAlone[0]);
+                if (npml) chain = std::max(chain, kFixed[1] + len * kAlone[1]);
+                work += c * (len + kStart) * (nin * kShared[0] + npml * kShared[1]);
+            }
+            const double t = chain + work / kSm;
+            if (best_t < 0.0 || t < 0.99 * best_t) {   // the longer lengths come first
+                best_t = t;
+                best = SegPlan{li, lp};
+            }
+        }
+    return best;
+}
+}  // namespace
+
 // Host-only plan of a 3D run's tiles: kTile3X x kTile3Y columns, a segment
-// of up to kSeg3 planes each; a tile takes the CPML instantiation if any cell
-// it updates or recomputes (one halo cell in x and y, the plane below the
-// segment) lies within one cell of an absorbing slab along any axis.  z
-// segments of at most kSeg3 planes never mix planes near a z slab with planes
-// away from it, so only the planes that need CPML code run it.  Needs no
-// device; orf_plan3d exposes it for checks of the tiling.
+// of up to kSeg3 planes each (seg_lengths); a tile takes the CPML
+// instantiation if any cell it updates or recomputes (one halo cell in x and
+// y, the plane below the segment) lies within one cell of an absorbing slab
+// along any axis.  z segments never mix planes near a z slab with planes away
+// from it, so only the planes that need CPML code run it.  Needs no device;
+// orf_plan3d exposes it for checks of the tiling.
 void plan3d(const orf_sim3d* s, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml, bool zlo, bool zhi) {
     const int n[3] = {s->nx, s->ny, s->nz};
     bool per[3];
@@ -140,13 +184,31 @@ void plan3d(const orf_sim3d* s, std::vector<Tile3D>& tiles, std::vector<Tile3D>&
         const bool at_lo = q != 2 || zlo, at_hi = q != 2 || zhi;
         return (at_lo && lo < np + 1) || (at_hi && hi > n[q] - np - 2);
     };
-    std::vector<std::pair<int, int>> segs;
+    // the columns near an x / y slab, and the runs of planes near a z slab or
+    // away from both
+    int cols_in = 0, cols_pml = 0;
+    for (int j0 = 0; j0 < n[1]; j0 += kTile3Y)
+        for (int i0 = 0; i0 < n[0]; i0 += kTile3X) {
+            const bool pm = near_pml(0, i0 - 1, std::min(i0 + kTile3X, n[0]) + 1) ||
+                            near_pml(1, j0 - 1, std::min(j0 + kTile3Y, n[1]) + 1);
+            ++(pm ? cols_pml : cols_in);
+        }
+    std::vector<std::pair<int, bool>> zones;
     for (int k0 = 0; k0 < n[2];) {
         const bool pz0 = near_pml(2, k0 - 1, k0 + 2);
         int k1 = k0 + 1;
-        while (k1 < n[2] && k1 - k0 < kSeg3 && near_pml(2, k1 - 1, k1 + 2) == pz0) ++k1;
-        segs.push_back({k0, k1});
+        while (k1 < n[2] && near_pml(2, k1 - 1, k1 + 2) == pz0) ++k1;
+        zones.push_back({k1 - k0, pz0});
         k0 = k1;
+    }
+    const SegPlan len = seg_lengths(cols_in, cols_pml, zones);
+    std::vector<std::pair<int, int>> segs;
+    int z0 = 0;
+    for (auto [planes, pz0] : zones) {   // equal segments
+        const int c = (planes + (pz0 ? len.pml : len.in) - 1) / (pz0 ? len.pml : len.in);
+        for (int q = 0; q < c; ++q)
+            segs.push_back({z0 + (int)((int64_t)planes * q / c), z0 + (int)((int64_t)planes * (q + 1) / c)});
+        z0 += planes;
     }
     for (auto [k0, k1] : segs)
         for (int j0 = 0; j0 < n[1]; j0 += kTile3Y)

@@ -200,3 +200,20 @@ def test_random_3d_plans(seed):
 def test_pillar_lattice_3d_plan():
     p = _check3d(_sim3d((600, 600, 300), (0, 0, 20), (True, True, False)))
     assert p["n_interior"] > 0 and p["n_cpml"] > 0
+
+
+@pytest.mark.parametrize("n,npml,per,longest", [
+    ((22, 22, 171), (0, 0, 12), (True, True, False), 8),     # three columns: short segments
+    ((14, 2, 60), (0, 0, 3), (True, True, False), 6),        # one column
+    ((201, 93, 77), (8, 8, 8), (False, False, False), 16),   # a grid of about one CTA slot per segment
+    ((600, 600, 300), (0, 0, 20), (True, True, False), 60),  # a grid that fills the SMs keeps long ones
+])
+def test_3d_segments_fit_the_grid(n, npml, per, longest):
+    """Small grids are marched in short z segments, large ones in long ones;
+    the segments of a run of planes differ by at most one plane."""
+    t = _check3d(_sim3d(n, npml, per))["tiles"]
+    length = t["k1"] - t["k0"]
+    assert longest / 2 < np.max(length[t["kind"] == 0]) <= longest
+    first = (t["i0"] == 0) & (t["j0"] == 0)
+    inner = first & (t["k0"] > npml[2] + 1) & (t["k1"] < n[2] - npml[2] - 2)
+    assert np.ptp(length[inner]) <= 1
