@@ -461,8 +461,10 @@ ORF_API int32_t orf_eps3d(orf_ctx* ctx, const double* x, const double* y, const 
  * stretched-coordinate PML s = 1 + i a (depth/L)^3 (e^{-i w t} convention)
  * of npml cells per side, a = 2 ln(1/R) / (k0 L), L = npml dx.
  * orf_fdfd2d_factor builds the operator and factors it on the device (block
- * LU along the longer axis; the shorter axis may hold at most 384 points);
- * each orf_fdfd2d_solve is then one forward and one backward sweep.
+ * LU along the longer axis, cut into segments eliminated side by side; the
+ * shorter axis may hold at most 384 points); each orf_fdfd2d_solve is then
+ * sweeps over the segments and the lines between them, with a step of
+ * iterative refinement.
  * Complex arrays are interleaved (re, im) pairs of nx*nz entries in
  * column-major order (entry (i, k) at i + nx*k), as MATLAB's interleaved
  * complex API hands them over. */

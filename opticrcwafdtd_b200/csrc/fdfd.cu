@@ -5,29 +5,39 @@
 //
 // on the FDTD's E_y points, E = 0 outside the grid, stretched-coordinate PML
 // s = 1 + i a (depth / L)^3 (e^{-i w t}), discretised with the 5-point
-// stencil.  Ordered block by block along the longer axis, the matrix is block
+// stencil.  Ordered line by line along the longer axis, the matrix A is block
 // tridiagonal: blocks of m = min(nx, nz) unknowns (one line across the
 // shorter axis), tridiagonal diagonal blocks, diagonal couplings to the
-// neighbouring lines.  The factorisation is the block LU of that structure,
-//   D_0 = A_00,  D_b = A_bb - B_b D_{b-1}^{-1} C_{b-1},
-// with every D_b inverted by Gauss-Jordan elimination with partial pivoting
-// and the inverses kept on the device; a solve is then a forward and a
-// backward sweep of matrix-vector products with them (m^2 per line), for A
-// and, with the same inverses, for A.' (the adjoint, fdfd2D.m:13-15).
+// neighbouring lines.  M = diag(s_x s_z) A is complex symmetric, and M is what
+// is factored: A E = -J is M E = -s J, and the adjoint A.' lam = g is
+// M u = g, lam = s u, so one set of factors and one kind of sweep serve both.
 //
-// The block inversions run on one thread-block cluster of 8 CTAs (16, a
-// non-portable cluster size, for blocks above 128 points): CTA c
-// holds rows [c R, c R + R) of the block in registers (one column per
-// thread, the rows split over up to four thread groups).
-// At each pivot step every CTA stores its pivot candidate into the shared
-// memory of every CTA of the cluster; after a cluster barrier all pick the
-// same pivot, its owner stores the pivot row into every CTA (and the owner
-// of row k that row into the pivot row's owner), and after a second barrier
-// each CTA eliminates from local copies: no remote read, one row broadcast
-// per pivot.  The next block's Schur complement is formed from the
-// inverse while it is still in registers.  Cluster barriers are hardware
-// barriers: no CTA spins on memory.
+// Factorisation.  The lines are cut into S segments, with one separator line
+// between neighbours.  Each segment is eliminated line by line,
+//   D_0 = M_00,  D_b = M_bb - E_b D_{b-1}^{-1} E_b   (E_b: the line couplings),
+// by its own thread-block cluster, every D_b inverted and kept; the last
+// segment runs from its far end.  The separators' Schur complement is block
+// tridiagonal, with dense blocks made of the corner blocks of the segments'
+// inverses; those of the segments with two separators come from
+//   L_b = -D_b^{-1} E_b L_{b-1} ([last, first]),  F_b = F_{b-1} - L_b.' E_b L_{b-1}
+// ([first, first]) by matrix products over all segments at once.  The
+// separators are then eliminated from both ends towards the middle one.
+// A chain of nb inversions becomes one of about nb / S + S / 2: with one
+// segment (a cluster of 16 CTAs on 16 of the 148 SMs) the 501 x 221 guide took
+// 400 ms, with 15 segments of 8 CTAs 25.
+// A segment between two separators is a closed cavity and can be nearly
+// singular where the whole operator is not.  So a factorisation with several
+// segments is tried on one right-hand side: if the residual is not that of a
+// stable solve, the operator is factored again as one segment.  Each solve
+// checks its residual too and takes a step of refinement where it is above
+// rounding.
+//
+// A solve is a forward and a backward sweep of every segment (for the
+// separators' right-hand side), the separators' two sweeps, and a second pair
+// of segment sweeps with the separators' values known.
 #include <cooperative_groups.h>
+
+#include <math_constants.h>
 
 #include <complex>
 
@@ -39,25 +49,23 @@ namespace orf {
 namespace {
 
 constexpr int kFdMaxM = 384;      // largest block (the shorter grid axis)
-constexpr int kFdMaxC = 16;       // largest cluster
-constexpr int kSolveThreads = 256;
+constexpr unsigned kFull = 0xffffffffu;
 
 struct FdfdDev {
-    int m, nb;                 // block size, number of blocks
+    int m, nb;                 // block size, number of lines
     const double2* diag;       // [nb][m]
-    const double2* wm;         // [nb][m]: coupling to p - 1 inside the block
-    const double2* wp;         // [nb][m]: to p + 1
-    const double2* bm;         // [nb][m]: to the same p of block b - 1
-    const double2* bp;         // [nb][m]: to block b + 1
+    const double2* wc;         // [nb][m]: coupling of p - 1 and p inside the line (entry 0 unused)
+    const double2* eb;         // [nb][m]: coupling of line b - 1 and b at p (line 0 unused)
     double2* inv;              // [nb][m][m]: D_b^{-1}, row-major
     int* fault;                // a zero pivot (singular block)
-    double2* xpan;             // [m][kPanel]: the blocked factorisation's panel, every row
-    double2* xrow;             // [kPanel][m]: its pivot rows
+    double2* xrow;             // [clusters][kPanel][m]: pivot rows of a panel
 };
 
-struct FdCand {   // a CTA's pivot candidate: |value|^2 and row (m: none)
-    double v;
-    int i, pad;
+// Lines a .. a+n-1, eliminated upwards (dir 1) or downwards (dir -1); dense:
+// one line whose block is given as a matrix.
+struct FdSeg {
+    int a, n, dir, pad;
+    const double2* dense;
 };
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -66,444 +74,228 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
-
-// Block LU of the whole operator: block b inverted in place, stored to
-// P.inv[b], then turned into D_{b+1} = A - B D_b^{-1} C in registers.
-// Thread (j, h) = (t % mp, t / mp) holds column j of the CTA's rows
-// h*RS .. h*RS + RS - 1 (TPC groups of RS rows; mp = m rounded up to a warp),
-// so that a pivot step's row work is spread over TPC times as many warps.
-template <int RS, int TPC, int NT>
-__global__ void __launch_bounds__(NT, 1) k_fdfd_factor(FdfdDev P) {
-    constexpr int RM = RS * TPC;   // rows per CTA at most
-    cg::cluster_group cl = cg::this_cluster();
-    const int C = (int)cl.num_blocks();
-    const int c = (int)cl.block_rank();
-    const int m = P.m;
-    const int mp = (m + 31) / 32 * 32;
-    const int R = (m + C - 1) / C;
-    const int r0 = c * R;
-    const int nr = max(0, min(m, r0 + R) - r0);
-    const int t = threadIdx.x;
-    const int j = t % mp, h = t / mp;
-    const int q0 = h * RS;            // first of this thread's rows, local to the CTA
-    const int r1 = r0 + q0;           // ... as a row of the block
-    const int nq = max(0, min(RS, nr - q0));   // this thread's rows
-    const bool col = j < m;
-
-    // Exchange buffers, per pivot parity, written by the other CTAs of the
-    // cluster (remote stores before a cluster barrier) and read locally after
-    // it: every CTA's pivot candidate (|value|^2, row), the pivot row, and
-    // row k (sent to the pivot row's owner only).
-    __shared__ FdCand s_cv[2][kFdMaxC];
-    // s_prow[2] and s_rowk[2] in the pivot steps; the column exchange of a
-    // finished block (up to 4 row groups) reuses them: no CTA writes them
-    // again before the next block's first candidate barrier, which this CTA
-    // reaches only after its exchange
-    __shared__ double2 s_ex[4][kFdMaxM];
-    double2 (*s_prow)[kFdMaxM] = s_ex;
-    double2 (*s_rowk)[kFdMaxM] = s_ex + 2;
-    __shared__ double2 s_colk[2][RM];   // column k of the owned rows, before the exchange
-    __shared__ FdCand s_hc[2][TPC];     // the row groups' candidates
-    __shared__ int s_piv[kFdMaxM];
-    __shared__ int s_perm[kFdMaxM];
-    static_assert(TPC <= 4, "the column exchange uses s_ex");
-
-    double2 a[RS];
-#pragma unroll
-    for (int u = 0; u < RS; ++u) a[u] = make_double2(0.0, 0.0);
-    long long g = 0;   // pivot steps so far (buffer parity)
-
-    for (int b = 0; b < P.nb; ++b) {
-        // ---- D_b: the tridiagonal block minus B_b D_{b-1}^{-1} C_{b-1}
-        if (col) {
-            const double2 cpj = b > 0 ? P.bp[(size_t)(b - 1) * m + j] : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < RS; ++u) {
-                if (u >= nq) break;
-                const int p = r1 + u;
-                const size_t o = (size_t)b * m + p;
-                double2 v = make_double2(0.0, 0.0);
-                if (b > 0) {
-                    const double2 s = cmul(cmul(P.bm[o], a[u]), cpj);
-                    v = make_double2(-s.x, -s.y);
-                }
-                if (j == p) v = cadd(v, P.diag[o]);
-                else if (j == p - 1) v = cadd(v, P.wm[o]);
-                else if (j == p + 1) v = cadd(v, P.wp[o]);
-                a[u] = v;
-            }
-        }
-        // ---- Gauss-Jordan inversion in place, partial pivoting
-        for (int k = 0; k < m; ++k, ++g) {
-            const int par = (int)(g & 1);
-            if (j == k) {   // the group's candidate: the largest |a| of column k on its rows >= k
-                double best = -1.0;
-                int bi = m;
-#pragma unroll
-                for (int u = 0; u < RS; ++u) {
-                    if (q0 + u < RM) s_colk[par][q0 + u] = a[u];
-                    if (u >= nq) continue;
-                    const int r = r1 + u;
-                    const double v = cabs2(a[u]);
-                    if (r >= k && v > best) {
-                        best = v;
-                        bi = r;
-                    }
-                }
-                s_hc[par][h] = FdCand{best, bi, 0};
-            }
-            __syncthreads();
-            // the CTA's candidate (the same in every thread)
-            double cbest = -1.0;
-            int bl = m;
-#pragma unroll
-            for (int hh = 0; hh < TPC; ++hh) {
-                const FdCand cd = s_hc[par][hh];
-                if (cd.i < m && (cd.v > cbest || (cd.v == cbest && cd.i < bl))) {
-                    cbest = cd.v;
-                    bl = cd.i;
-                }
-            }
-            if (t == 0) {   // the CTA's candidate into every CTA
-                const FdCand cd{cbest, bl, 0};
-                for (int c2 = 0; c2 < C; ++c2) *cl.map_shared_rank(&s_cv[par][c], c2) = cd;
-            }
-            cl.sync();   // every CTA's candidate is here
-            // the pivot row: the largest candidate, the lowest row on a tie;
-            // lane c2 of every warp reads CTA c2's candidate and the warp
-            // reduces (every warp decides the same)
-            int p;
-            {
-                const int lane = t & 31;
-                double best = -1.0;
-                int bi = m;
-                if (lane < C) {
-                    const FdCand cd = s_cv[par][lane];
-                    if (cd.i < m) {
-                        best = cd.v;
-                        bi = cd.i;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ob > best || (ob == best && oi < bi)) {
-                        best = ob;
-                        bi = oi;
-                    }
-                }
-                p = bi;
-            }
-            if (col) {   // the pivot row into every CTA, row k into the pivot row's owner
-                const bool hasp = p >= r1 && p < r1 + nq, hask = p != k && k >= r1 && k < r1 + nq;
-                if (hasp || hask) {
-                    double2 vp = make_double2(0.0, 0.0), vk = make_double2(0.0, 0.0);
-#pragma unroll
-                    for (int u = 0; u < RS; ++u) {
-                        if (r1 + u == p) vp = a[u];
-                        if (r1 + u == k) vk = a[u];
-                    }
-                    if (hasp)
-                        for (int c2 = 0; c2 < C; ++c2) cl.map_shared_rank(&s_prow[par][0], c2)[j] = vp;
-                    if (hask) cl.map_shared_rank(&s_rowk[par][0], p / R)[j] = vk;
-                }
-            }
-            cl.sync();   // the pivot row (and, at its owner, row k) is here
-            const double2* prow_all = &s_prow[par][0];
-            const double2* rowk = &s_rowk[par][0];
-            const double2 pk = prow_all[k];
-            const double dd = cabs2(pk);
-            const double inv_dd = dd == 0.0 ? 0.0 : 1.0 / dd;
-            const double2 ip = make_double2(pk.x * inv_dd, -pk.y * inv_dd);
-            if (t == 0) {
-                s_piv[k] = p;
-                if (dd == 0.0) atomicExch(P.fault, 1);
-            }
-            if (col && nq > 0) {
-                const double2 prow = prow_all[j];
-                const double2 pr = j == k ? ip : cmul(prow, ip);   // the scaled pivot row
-                const bool swap = p != k && p >= r1 && p < r1 + nq;   // row p takes the old row k
-                const double2 rkj = rowk[j], rkk = rowk[k];
-#pragma unroll
-                for (int u = 0; u < RS; ++u) {
-                    if (u >= nq) break;
-                    const int r = r1 + u;
-                    if (r == k) {
-                        a[u] = pr;
-                    } else {
-                        // column k of the inverse: -f / pivot (pr = 1 / pivot there)
-                        const bool sw = swap && r == p;
-                        const double2 f = sw ? rkk : s_colk[par][q0 + u];
-                        const double2 cur = j == k ? make_double2(0.0, 0.0) : (sw ? rkj : a[u]);
-                        a[u] = csub(cur, cmul(f, pr));
-                    }
-                }
-            }
-        }
-        // ---- undo the row exchanges on the columns of the inverse, last first:
-        // column j of D_b^{-1} is column perm[j] of what the threads hold
-        __syncthreads();
-        if (t == 0) {
-            for (int q = 0; q < m; ++q) s_perm[q] = q;
-            for (int k = m - 1; k >= 0; --k) {
-                const int pk = s_piv[k];
-                if (pk != k) {
-                    const int tmp = s_perm[k];
-                    s_perm[k] = s_perm[pk];
-                    s_perm[pk] = tmp;
-                }
-            }
-        }
-        __syncthreads();
-        const int src = col ? s_perm[j] : 0;
-#pragma unroll
-        for (int u = 0; u < RS; ++u) {
-            if (col) s_ex[h][j] = a[u];
-            __syncthreads();
-            if (col) a[u] = s_ex[h][src];
-            __syncthreads();
-        }
-        if (col) {
-            double2* out = P.inv + (size_t)b * m * m;
-#pragma unroll
-            for (int u = 0; u < RS; ++u) {
-                if (u >= nq) break;
-                out[(size_t)(r1 + u) * m + j] = a[u];
-            }
-        }
-    }
-    cl.sync();   // no CTA leaves while another may still read its shared memory
+// c + a b and c - a b
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
+    return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
+__device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 c) {
+    return make_double2(fma(-a.x, b.x, fma(a.y, b.y, c.x)), fma(-a.x, b.y, fma(-a.y, b.x, c.y)));
 }
 
-// Blocked form of the same elimination for blocks of up to 256 points:
-// pivots chosen and applied kPanel columns at a time.  Every CTA reads the
-// panel columns of all rows (each CTA writes its rows' entries to a global
-// scratch panel, cluster barrier, every CTA reads it back from L2: the
-// fan-out goes through L2, not through one SM's port), runs the panel's
-// pivot steps on that copy with block barriers only (pivot rows by partial
-// pivoting among the rows not yet used, the lowest row on a tie: every CTA
-// decides the same), reads the panel's pivot rows the same way (second
-// cluster barrier), and applies the rank-kPanel update
-//   pivot rows:  A[K, N] <- P^-1 A[K, N],   others: A[r, N] -= A[r, K0] P^-1 A[K, N]
-// to its own rows (P: the panel block of the pivot rows, N: the columns
-// outside the panel); the panel columns take the replica's values.  Rows
-// are not exchanged: the inverse is the result with its rows taken in pivot
-// order and its columns in the inverse order, and is stored to P.inv row by
-// row in its true place, then read back for the next block.
+// Block inversions by Gauss-Jordan elimination with partial pivoting, blocked:
+// pivots are chosen and applied kPanel columns at a time.  CTA c of a cluster
+// holds rows [c R, c R + R) of the block in registers (thread (j, h) holds
+// column j of the rows of group h).  Per panel:
+//   - every CTA pushes its rows' entries of the panel columns into the shared
+//     memory of every CTA of the cluster (cluster barrier);
+//   - every CTA runs the panel's pivot steps on that copy (thread r holds row
+//     r; the pivot is the row of largest magnitude not yet used, compared on
+//     the leading 32 bits of |.|^2, the lowest row on a tie: every CTA decides
+//     the same).  A step is one barrier of the warps that hold rows: each warp
+//     publishes its candidate row, every warp picks the best of them;
+//   - the owners write the panel's pivot rows (old values, every column) to a
+//     global scratch and, after a second cluster barrier, every CTA reads them
+//     (from L2: the fan-out of up to eight whole rows would go through one
+//     SM's port);
+//   - the rank-kPanel update of the own rows, whose coefficients are what the
+//     pivot steps left in the copy's rows.
+// Rows are never exchanged: the inverse is the result with its rows in pivot
+// order and its columns in the inverse order, written row by row in its true
+// place and read back for the next line's Schur complement.
+// A panel of a 221-point block takes 12.7 us: the pivot steps 5.1 (0.64 each: the
+// reduction, a barrier, and the FP64 latency of a reciprocal and two products
+// in a row), the update 3.9 (FP64 units, a third of their rate), the two
+// exchanges 3.6.
 constexpr int kPanel = 8;
-constexpr int kPanelMaxM = 256;
 
-inline size_t fd_panel_smem(int m) {   // s_pan[m][W], s_pn[m][W], s_rk[W][m], s_u[W][m], s_rows[2][m][W]
-    return (size_t)6 * m * kPanel * sizeof(double2);
+inline size_t fd_factor_smem(int m, int R) {   // s_recv[2][m][W + 1], s_ex[4][m], s_own[R][W + 1], s_pn[R][W + 1]
+    return ((size_t)2 * (m + R) * (kPanel + 1) + (size_t)m * 4) * sizeof(double2);
 }
 
 template <int RS, int TPC, int NT>
-__global__ void __launch_bounds__(NT, 1) k_fdfd_factor_panel(FdfdDev P) {
+__global__ void __launch_bounds__(NT, 1) k_fdfd_factor(FdfdDev P, const FdSeg* __restrict__ segs) {
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks();
     const int c = (int)cl.block_rank();
+    const int cid = (int)(blockIdx.x / C);
+    const FdSeg seg = segs[cid];
     const int m = P.m;
     const int mp = (m + 31) / 32 * 32;
     const int R = (m + C - 1) / C;
     const int r0 = c * R;
     const int nr = max(0, min(m, r0 + R) - r0);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int nt = (int)blockDim.x, nwarps = nt / 32;   // TPC x mp threads (at most NT)
+    const int nt = (int)blockDim.x;                     // TPC x mp threads (at most NT)
+    const int nrw = mp / 32;                            // warps that hold rows of the panel copy
     const int j = t % mp, h = t / mp;
     const int q0 = h * RS;
     const int r1 = r0 + q0;
     const int nq = max(0, min(RS, nr - q0));
     const bool col = j < m;
-    constexpr int W = kPanel;
+    constexpr int W = kPanel, MW = kFdMaxM / 32, WP = W + 1;   // (rows of the copy padded: no bank conflicts)
+    double2* xrow = P.xrow + (size_t)cid * W * m;
+    // the push: thread t takes entries pq, pq + NPQ, .. for CTAs pc, pc + NPC, ..
+    constexpr int NPC = 2;
+    const int NPQ = nt / NPC, pq = t % NPQ, pc = t / NPQ;
 
     extern __shared__ double2 s_dyn[];
-    double2* s_pan = s_dyn;                          // [m][W]: the panel, every row (old values)
-    double2* s_pn = s_pan + (size_t)m * W;           // [m][W]: the panel after its pivot steps
-    double2* s_rk = s_pn + (size_t)m * W;            // [W][m]: the panel's pivot rows (old values)
-    double2* s_u = s_rk + (size_t)W * m;             // [W][m]: P^-1 times them
-    double2* s_rows = s_u + (size_t)W * m;           // [2][m][W]: the copy's rows, per pivot step
-    __shared__ FdCand s_wc[2][NT / 32];              // per warp candidates, per pivot step
-    __shared__ int s_K[W];                           // pivot rows of the panel
-    __shared__ signed char s_kidx[kPanelMaxM];       // index of a row in s_K, or -1
-    __shared__ int s_piv[kPanelMaxM];
-    __shared__ int s_ipiv[kPanelMaxM];
+    double2* s_recv = s_dyn;                         // [2][m][WP]: the panel columns, every row (old values)
+    double2* s_ex = s_recv + (size_t)2 * m * WP;     // [TPC][m]: exchange of a finished block's columns
+    double2* s_own = s_ex + (size_t)4 * m;            // [R][WP]: the own rows' panel entries, before the push
+    double2* s_pn = s_own + (size_t)R * WP;           // [R][WP]: the own rows' panel entries after the pivot steps
+    __shared__ double2 s_cand[2][MW][W];             // a warp's candidate row, by step parity
+    __shared__ int2 s_ckey[2][MW];                   // its key and row, 1 / |candidate|^2
+    __shared__ double s_cinv[2][MW];
+    __shared__ signed char s_kown[32];               // index among the panel's pivots of an own row, or -1
+    __shared__ int s_piv[kFdMaxM], s_ipiv[kFdMaxM];
 
     double2 a[RS];
 #pragma unroll
     for (int u = 0; u < RS; ++u) a[u] = make_double2(0.0, 0.0);
+    int par = 0;
 
-    for (int b = 0; b < P.nb; ++b) {
-        // ---- D_b: the tridiagonal block minus B_b D_{b-1}^{-1} C_{b-1}
+    for (int it = 0; it < seg.n; ++it) {
+        const int b = seg.dir > 0 ? seg.a + it : seg.a + seg.n - 1 - it;
         if (col) {
-            const double2 cpj = b > 0 ? P.bp[(size_t)(b - 1) * m + j] : make_double2(0.0, 0.0);
+            const double2* e = P.eb + (size_t)(seg.dir > 0 ? b : b + 1) * m;   // to the line before (it > 0)
+            const double2 ej = it > 0 ? e[j] : make_double2(0.0, 0.0);
 #pragma unroll
             for (int u = 0; u < RS; ++u) {
                 if (u >= nq) break;
                 const int p = r1 + u;
+                if (seg.dense) {
+                    a[u] = seg.dense[(size_t)p * m + j];
+                    continue;
+                }
                 const size_t o = (size_t)b * m + p;
                 double2 v = make_double2(0.0, 0.0);
-                if (b > 0) {
-                    const double2 s = cmul(cmul(P.bm[o], a[u]), cpj);
+                if (it > 0) {
+                    const double2 s = cmul(cmul(e[p], a[u]), ej);
                     v = make_double2(-s.x, -s.y);
                 }
                 if (j == p) v = cadd(v, P.diag[o]);
-                else if (j == p - 1) v = cadd(v, P.wm[o]);
-                else if (j == p + 1) v = cadd(v, P.wp[o]);
+                else if (j == p - 1) v = cadd(v, P.wc[o]);
+                else if (j == p + 1) v = cadd(v, P.wc[o + 1]);
                 a[u] = v;
             }
         }
         bool myused = false;   // row t (thread t < m) is the pivot row of an earlier column
-        for (int k0 = 0; k0 < m; k0 += W) {
+        for (int k0 = 0; k0 < m; k0 += W, par ^= 1) {
             const int we = min(W, m - k0);
-            double2* pan = s_pan;
-            // ---- the panel entries of the own rows to the scratch panel; every
-            // CTA reads the whole panel back (L2, bypassing L1: the scratch is
-            // rewritten every panel).  The scratch is written again only after
-            // the next cluster barrier, which every reader reaches after its read.
-            if (col && j >= k0 && j < k0 + we) {
+            double2* pan = s_recv + (size_t)par * m * WP;
+            // ---- the panel entries of the own rows into every CTA of the
+            // cluster.  (Buffer par was last read in the update two panels ago;
+            // every CTA has since passed a cluster barrier of the panel before.)
+            // (columns past the last one are zero)
+            if (j >= k0 && j < k0 + W) {
 #pragma unroll
                 for (int u = 0; u < RS; ++u)
-                    if (u < nq) P.xpan[(size_t)(r1 + u) * W + (j - k0)] = a[u];
-            }
-            __threadfence();
-            cl.sync();   // the whole panel is in memory
-            // ---- the panel's pivot steps on the copy: thread r holds row r
-            double2 pr[W];
-            if (t < m) {
-#pragma unroll
-                for (int l = 0; l < W; ++l) {
-                    pr[l] = l < we ? __ldcg(P.xpan + (size_t)t * W + l) : make_double2(0.0, 0.0);
-                    pan[(size_t)t * W + l] = pr[l];
-                }
-            }
-            // one block barrier per pivot step: every row thread publishes its
-            // row and every warp its candidate (buffers alternate by step), then
-            // every warp reduces the candidates itself and reads the pivot row
-            // (unrolled: a row's entries are registers indexed by the step)
-#pragma unroll
-            for (int aa = 0; aa < W; ++aa) {
-                if (aa >= we) break;
-                const int sp2 = aa & 1;
-                double2* rows = s_rows + (size_t)sp2 * m * W;
-                double best = -1.0;
-                int bi = m;
-                if (t < m) {
-#pragma unroll
-                    for (int l = 0; l < W; ++l) rows[(size_t)t * W + l] = pr[l];
-                    if (!myused) {
-                        best = cabs2(pr[aa]);
-                        bi = t;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ob > best || (ob == best && oi < bi)) {
-                        best = ob;
-                        bi = oi;
-                    }
-                }
-                if (lane == 0) s_wc[sp2][warp] = FdCand{best, bi, 0};
-                __syncthreads();
-                best = -1.0;
-                bi = m;
-                if (lane < nwarps) {
-                    const FdCand cd = s_wc[sp2][lane];
-                    best = cd.v;
-                    bi = cd.i;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ob > best || (ob == best && oi < bi)) {
-                        best = ob;
-                        bi = oi;
-                    }
-                }
-                const bool bad = bi >= m || best == 0.0;
-                const int p = bi >= m ? 0 : bi;
-                if (t == 0) {
-                    if (bad) atomicExch(P.fault, 1);
-                    s_piv[k0 + aa] = p;
-                    s_K[aa] = p;
-                }
-                if (t == p) myused = true;
-                const double2* prw = rows + (size_t)p * W;
-                const double2 pk = prw[aa];
-                const double dd = cabs2(pk);
-                const double inv_dd = dd == 0.0 ? 0.0 : 1.0 / dd;
-                const double2 ip = make_double2(pk.x * inv_dd, -pk.y * inv_dd);
-                if (t < m) {
-                    const double2 f = pr[aa];
-#pragma unroll
-                    for (int l = 0; l < W; ++l) {
-                        const double2 sp = l == aa ? ip : cmul(prw[l], ip);   // the scaled pivot row
-                        if (t == p) pr[l] = sp;
-                        else pr[l] = csub(l == aa ? make_double2(0.0, 0.0) : pr[l], cmul(f, sp));
-                    }
-                }
-            }
-            __syncthreads();   // s_K, s_piv
-            if (t < m) {
-#pragma unroll
-                for (int l = 0; l < W; ++l) s_pn[(size_t)t * W + l] = pr[l];
-                s_kidx[t] = -1;
+                    if (u < nq) s_own[(q0 + u) * WP + (j - k0)] = col ? a[u] : make_double2(0.0, 0.0);
             }
             __syncthreads();
-            if (t < we) s_kidx[s_K[t]] = (signed char)t;
+            for (int q = pq; q < nr * WP; q += NPQ)
+                for (int c2 = pc; c2 < C; c2 += NPC) cl.map_shared_rank(pan, c2)[r0 * WP + q] = s_own[q];
+            cl.sync();   // the whole panel is here
+            // ---- the panel's pivot steps on the copy: thread r holds row r
+            if (warp < nrw) {
+                double2 pr[W];
+                int myk = -1;
+#pragma unroll
+                for (int l = 0; l < W; ++l) pr[l] = t < m ? pan[t * WP + l] : make_double2(0.0, 0.0);
+#pragma unroll
+                for (int aa = 0; aa < W; ++aa) {
+                    if (aa >= we) break;
+                    const int sp = aa & 1;
+                    // (the sign bit cleared: a NaN has a key too, and every row is
+                    // used once; every row forms its reciprocal while the warps agree)
+                    const double dd = cabs2(pr[aa]);
+                    const int key = t < m && !myused ? __double2hiint(dd) & 0x7fffffff : -1;
+                    const int wkey = __reduce_max_sync(kFull, key);
+                    const double inv_dd = dd == 0.0 ? 0.0 : 1.0 / dd;
+                    const int wl = __ffs(__ballot_sync(kFull, key == wkey)) - 1;
+                    if (lane == wl) {
+                        s_ckey[sp][warp] = make_int2(wkey, t);
+                        s_cinv[sp][warp] = inv_dd;
+#pragma unroll
+                        for (int l = 0; l < W; ++l) s_cand[sp][warp][l] = pr[l];
+                    }
+                    asm volatile("bar.sync 1, %0;" ::"r"(32 * nrw) : "memory");   // the row warps
+                    const int2 ck = lane < nrw ? s_ckey[sp][lane] : make_int2(-2, 0);
+                    const int bk = __reduce_max_sync(kFull, ck.x);
+                    const int bw = __ffs(__ballot_sync(kFull, ck.x == bk)) - 1;
+                    const int p = __shfl_sync(kFull, ck.y, bw);
+                    const double2* prw = s_cand[sp][bw];
+                    const double pinv = s_cinv[sp][bw];
+                    const double2 ip = make_double2(prw[aa].x * pinv, -prw[aa].y * pinv);   // 1 / pivot
+                    if (t == 0) s_piv[k0 + aa] = p;
+                    // others: row -= (f / pivot) pivot row; the pivot row: divided by the pivot
+                    const bool me = t == p;
+                    double2 g = cmul(pr[aa], ip);
+                    g = me ? ip : make_double2(-g.x, -g.y);
+                    myused = myused || me;
+                    myk = me ? aa : myk;
+#pragma unroll
+                    for (int l0 = 1; l0 < W; ++l0) {   // the next step's column first
+                        const int l = (aa + l0) % W;
+                        const double2 base = me ? make_double2(0.0, 0.0) : pr[l];
+                        pr[l] = cfma(g, prw[l], base);
+                    }
+                    pr[aa] = g;
+                    if (me && dd == 0.0) atomicExch(P.fault, 1);   // a zero pivot
+                }
+                if (t >= r0 && t < r0 + nr) {
+                    s_kown[t - r0] = (signed char)myk;
+#pragma unroll
+                    for (int l = 0; l < W; ++l) s_pn[(t - r0) * WP + l] = pr[l];
+                }
+            }
+            __syncthreads();
             // ---- the panel's pivot rows (old values, every column) through the
-            // scratch rows, read back by every CTA
+            // scratch rows.  (They were last read before this panel's first
+            // cluster barrier.)
             if (col) {
 #pragma unroll
                 for (int u = 0; u < RS; ++u) {
                     if (u >= nq) break;
-                    const int r = r1 + u;
-                    for (int i = 0; i < we; ++i)
-                        if (s_K[i] == r) P.xrow[(size_t)i * m + j] = a[u];
+                    const int ki = s_kown[q0 + u];
+                    if (ki >= 0) __stcg(xrow + (size_t)ki * m + j, a[u]);
                 }
             }
             __threadfence();
             cl.sync();   // the pivot rows are in memory
-            for (int e = t; e < we * m; e += nt) s_rk[e] = __ldcg(P.xrow + e);
-            __syncthreads();
-            // ---- U = P^-1 (pivot rows): row i of U by the threads of group i % TPC
+            // ---- the rank-kPanel update of the own rows, four at a time: after
+            // the pivot steps the copy's entries of a row are the coefficients
+            // of the pivot rows in its update, P^-1 for a pivot row (whose old
+            // values count for nothing more) and -A[r, K0] P^-1 for the others
             if (col) {
-                for (int i = h; i < we; i += TPC) {
-                    double2 acc = make_double2(0.0, 0.0);
-                    const double2* pinv = s_pn + (size_t)s_K[i] * W;
-                    for (int l = 0; l < we; ++l) acc = cadd(acc, cmul(pinv[l], s_rk[(size_t)l * m + j]));
-                    s_u[(size_t)i * m + j] = acc;
-                }
-            }
-            __syncthreads();
-            // ---- the rank-we update of the own rows
-            if (col) {
+                double2 rk[W];
+#pragma unroll
+                for (int l = 0; l < W; ++l) rk[l] = l < we ? __ldcg(xrow + l * m + j) : make_double2(0.0, 0.0);
                 const bool inpan = j >= k0 && j < k0 + we;
 #pragma unroll
-                for (int u = 0; u < RS; ++u) {
-                    if (u >= nq) break;
-                    const int r = r1 + u;
+                for (int u0 = 0; u0 < RS; u0 += 4) {
+                    if (u0 >= nq) break;
+#pragma unroll
+                    for (int u = u0; u < u0 + 4; ++u)
+                        if (s_kown[min(q0 + u, R - 1)] >= 0) a[u] = make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int l = 0; l < W; ++l)
+#pragma unroll
+                        for (int u = u0; u < u0 + 4; ++u)   // (rows past nq: values never used)
+                            a[u] = cfma(s_pn[min(q0 + u, R - 1) * WP + l], rk[l], a[u]);
                     if (inpan) {
-                        a[u] = s_pn[(size_t)r * W + (j - k0)];
-                    } else if (s_kidx[r] >= 0) {
-                        a[u] = s_u[(size_t)s_kidx[r] * m + j];
-                    } else {
-                        double2 v = a[u];
-                        for (int l = 0; l < we; ++l) v = csub(v, cmul(pan[(size_t)r * W + l], s_u[(size_t)l * m + j]));
-                        a[u] = v;
+#pragma unroll
+                        for (int u = u0; u < u0 + 4; ++u) a[u] = s_pn[min(q0 + u, R - 1) * WP + (j - k0)];
                     }
                 }
             }
-            __syncthreads();   // s_kidx, s_u and s_pn are rewritten by the next panel
         }
         // ---- the inverse: row ipiv[r] is row r of what the threads hold,
         // with column j taken from column ipiv[j]
+        __syncthreads();
         if (t < m) s_ipiv[s_piv[t]] = t;
         __syncthreads();
-        double2* s_ex = s_u;   // [TPC][m] (TPC <= kPanel)
+        static_assert(TPC <= 4, "s_ex");
         const int src = col ? s_ipiv[j] : 0;
 #pragma unroll
         for (int u = 0; u < RS; ++u) {
@@ -516,161 +308,487 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_factor_panel(FdfdDev P) {
         if (col) {
 #pragma unroll
             for (int u = 0; u < RS; ++u)
-                if (u < nq) out[(size_t)s_ipiv[r1 + u] * m + j] = a[u];
+                if (u < nq) __stcg(out + (size_t)s_ipiv[r1 + u] * m + j, a[u]);
         }
-        __threadfence();
-        cl.sync();   // every CTA's rows of the inverse are in memory
-        if (col) {
+        if (it + 1 < seg.n) {
+            __threadfence();
+            cl.sync();   // every CTA's rows of the inverse are in memory
+            if (col) {
 #pragma unroll
-            for (int u = 0; u < RS; ++u)
-                if (u < nq) a[u] = out[(size_t)(r1 + u) * m + j];
+                for (int u = 0; u < RS; ++u)
+                    if (u < nq) a[u] = __ldcg(out + (size_t)(r1 + u) * m + j);
+            }
         }
-        __syncthreads();
     }
-    cl.sync();   // no CTA leaves while another may still read its shared memory
+    cl.sync();   // no CTA leaves while another may still write its shared memory
 }
 
-// Forward and backward sweeps with the stored inverses.
-//   mode 0: A x = -rhs:   w_b = -rhs_b - B_b y_{b-1},  y_b = D_b^{-1} w_b,
-//                         x_b = y_b - D_b^{-1} C_b x_{b+1}
-//   mode 1: A.' x = rhs:  z_b = D_b^{-T} (rhs_b - C_{b-1} z_{b-1}),
-//                         x_{b-1} = z_{b-1} - D_{b-1}^{-T} B_b x_b
-// Vector entries are owned by the CTA that owns the row of the same index;
-// the products gather the whole vector (mode 0) or reduce partial sums over
-// the owned rows (mode 1) through distributed shared memory, one cluster
-// barrier per line.
-__global__ void __launch_bounds__(kSolveThreads, 1) k_fdfd_solve(FdfdDev P, const double2* rhs, double2* x,
-                                                                  double2* Y, int mode) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int C = (int)cl.num_blocks();
-    const int c = (int)cl.block_rank();
-    const int m = P.m, nb = P.nb;
-    const int R = (m + C - 1) / C;
-    const int r0 = c * R;
-    const int nr = max(0, min(m, r0 + R) - r0);
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    constexpr int NW = kSolveThreads / 32;
-    __shared__ double2 s_pub[2][kFdMaxM];   // published own entries (mode 0) / partial sums (mode 1)
-    __shared__ double2 s_full[kFdMaxM];     // mode 0: the gathered vector
-    __shared__ double2 s_u[kFdMaxM];        // mode 1: the owned entries of the multiplied vector
-    long long g = 0;
-    auto warp_sum = [&](double2 v) {
+// C = C0 + sign op(A) diag(e) op(B) of m x m complex matrices, a batch of
+// problems per launch (blockIdx.z): 32 x 32 tiles by 128 threads, 2 x 4 results
+// a thread, the next 8 columns of op(A) and rows of op(B) loaded into registers
+// while the current ones (two shared buffers, one barrier a round) are
+// multiplied.  Bound by the FP64 units and, for one or two problems, by a
+// tile's own chain of rounds: 28 problems of 221^2 in 0.15 ms (16 TFLOP/s), one in 38 us.
+struct FdGemm {
+    const double2 *A, *B, *C0, *e;   // C0 null: zero; e null: ones
+    double2* C;
+    int ta, tb;                      // op is the transpose
+    double sign;
+};
+constexpr int kGT = 32, kGK = 8, kGN = 128;
+__global__ void __launch_bounds__(kGN) k_fd_gemm(const FdGemm* __restrict__ probs, int m) {
+    const FdGemm g = probs[blockIdx.z];
+    __shared__ double2 As[2][kGK][kGT + 1], Bs[2][kGK][kGT + 1];
+    constexpr int NL = kGT * kGK / kGN;   // loads of each operand per thread and round
+    const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
+    const int i0 = blockIdx.y * kGT, j0 = blockIdx.x * kGT;
+    const double2 zero = make_double2(0.0, 0.0);
+    // element (k, i) of op(A) and (k, j) of op(B), the fast index along memory
+    int ka[NL], ia[NL], kb[NL], jb[NL];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    for (int s = 0; s < NL; ++s) {
+        const int e = t + kGN * s;
+        ka[s] = g.ta ? e / kGT : e % kGK;
+        ia[s] = g.ta ? e % kGT : e / kGK;
+        kb[s] = g.tb ? e % kGK : e / kGT;
+        jb[s] = g.tb ? e / kGK : e % kGT;
+    }
+    double2 ra[NL], rb[NL];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int s = 0; s < NL; ++s) {
+            const int k = k0 + ka[s], i = i0 + ia[s];
+            ra[s] = i < m && k < m ? __ldg(g.ta ? g.A + (size_t)k * m + i : g.A + (size_t)i * m + k) : zero;
         }
-        return v;
+#pragma unroll
+        for (int s = 0; s < NL; ++s) {
+            const int k = k0 + kb[s], j = j0 + jb[s];
+            const bool v = j < m && k < m;
+            rb[s] = v ? __ldg(g.tb ? g.B + (size_t)j * m + k : g.B + (size_t)k * m + j) : zero;
+            if (g.e && v) rb[s] = cmul(rb[s], __ldg(g.e + k));
+        }
     };
-    if (mode == 0) {
-        // dst_b = D_b^{-1} s_full on the owned rows (base_b minus it when base is given)
-        auto gemv_rows = [&](int b, const double2* base, double2* dst) {
-            const double2* Ib = P.inv + (size_t)b * m * m;
-            for (int q = warp; q < nr; q += NW) {
-                const int p = r0 + q;
-                const double2* row = Ib + (size_t)p * m;
-                double2 acc = make_double2(0.0, 0.0);
-                for (int jj = lane; jj < m; jj += 32) acc = cadd(acc, cmul(row[jj], s_full[jj]));
-                acc = warp_sum(acc);
-                if (lane == 0) dst[(size_t)b * m + p] = base ? csub(base[(size_t)b * m + p], acc) : acc;
-            }
-        };
-        for (int b = 0; b < nb; ++b, ++g) {
-            const int par = (int)(g & 1);
-            for (int q = t; q < nr; q += kSolveThreads) {
-                const int p = r0 + q;
-                const size_t o = (size_t)b * m + p;
-                double2 w = make_double2(-rhs[o].x, -rhs[o].y);
-                if (b > 0) w = csub(w, cmul(P.bm[o], Y[o - m]));
-                s_pub[par][p] = w;
-            }
-            cl.sync();
-            for (int jj = t; jj < m; jj += kSolveThreads) s_full[jj] = cl.map_shared_rank(&s_pub[par][0], jj / R)[jj];
-            __syncthreads();
-            gemv_rows(b, nullptr, Y);
-            __syncthreads();
+    double2 acc[2][4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[r][q] = zero;
+    fetch(0);
+    int buf = 0;
+    for (int k0 = 0; k0 < m; k0 += kGK, buf ^= 1) {
+#pragma unroll
+        for (int s = 0; s < NL; ++s) {
+            As[buf][ka[s]][ia[s]] = ra[s];
+            Bs[buf][kb[s]][jb[s]] = rb[s];
         }
-        for (int q = t; q < nr; q += kSolveThreads) {
-            const size_t o = (size_t)(nb - 1) * m + r0 + q;
-            x[o] = Y[o];
+        __syncthreads();   // (the other buffer was read in the round before last's compute, a barrier ago)
+        if (k0 + kGK < m) fetch(k0 + kGK);
+#pragma unroll
+        for (int k = 0; k < kGK; ++k) {
+            double2 av[2], bv[4];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) av[r] = As[buf][k][ty + 16 * r];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bv[q] = Bs[buf][k][tx + 8 * q];
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[r][q] = cfma(av[r], bv[q], acc[r][q]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = i0 + ty + 16 * r, j = j0 + tx + 8 * q;
+            if (i >= m || j >= m) continue;
+            const size_t o = (size_t)i * m + j;
+            const double2 v = make_double2(g.sign * acc[r][q].x, g.sign * acc[r][q].y);
+            g.C[o] = g.C0 ? cadd(g.C0[o], v) : v;
+        }
+}
+
+// The separators' system: Kd[j] = M_jj - E [last, last] E - E [first, first] E
+// and T[j] = -E L E (the block of separators j and j-1), one row per block.
+struct FdSepIn {
+    int line;                        // the separator's line
+    int hasT;
+    const double2 *last, *first;     // corner blocks of the segments before and after
+    const double2* L;                // [last, first] of the segment before (hasT)
+};
+__global__ void k_fd_assemble(FdfdDev P, const FdSepIn* __restrict__ sep, double2* Kd, double2* T) {
+    const int m = P.m, q = blockIdx.y, p = blockIdx.x;
+    const FdSepIn s = sep[q];
+    const double2 *e0 = P.eb + (size_t)s.line * m, *e1 = e0 + m;   // couplings to the line before and after
+    const double2* ea = s.hasT ? P.eb + (size_t)(sep[q - 1].line + 1) * m : nullptr;
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const size_t o = (size_t)p * m + j;
+        double2 v = make_double2(0.0, 0.0);
+        if (j == p) v = P.diag[(size_t)s.line * m + p];
+        else if (j == p - 1) v = P.wc[(size_t)s.line * m + p];
+        else if (j == p + 1) v = P.wc[(size_t)s.line * m + p + 1];
+        v = csub(v, cmul(cmul(e0[p], s.last[o]), e0[j]));
+        v = csub(v, cmul(cmul(e1[p], s.first[o]), e1[j]));
+        Kd[(size_t)q * m * m + o] = v;
+        if (s.hasT) {
+            const double2 w = cmul(cmul(e0[p], s.L[o]), ea[j]);
+            T[(size_t)q * m * m + o] = make_double2(-w.x, -w.y);
+        }
+    }
+}
+__global__ void k_fd_transpose(const double2* __restrict__ a, double2* __restrict__ b, int m) {
+    __shared__ double2 s[16][17];
+    const size_t o = (size_t)blockIdx.z * m * m;
+    int i = blockIdx.y * 16 + threadIdx.y, j = blockIdx.x * 16 + threadIdx.x;
+    if (i < m && j < m) s[threadIdx.y][threadIdx.x] = a[o + (size_t)i * m + j];
+    __syncthreads();
+    i = blockIdx.x * 16 + threadIdx.y;
+    j = blockIdx.y * 16 + threadIdx.x;
+    if (i < m && j < m) b[o + (size_t)i * m + j] = s[threadIdx.x][threadIdx.y];
+}
+
+// Products of m x m matrices with vectors by a cluster: CTA c owns the rows
+// (and the vector entries) [c R, c R + R), warp w of it the rows w, w + NT/32,
+// .., a lane NQ columns of each.  A matrix's rows wait in registers, loaded
+// before the vector is known; the vector's entries are pushed into the shared
+// memory of every CTA (one cluster barrier per product).
+template <int NQ, int RW, int NT>
+struct FdMv {
+    static constexpr int NW = NT / 32;
+    int m, R, r0, nr, lane, warp;
+    double2 M[RW][NQ];
+    __device__ void load(const double2* __restrict__ A) {   // A: [m][m]
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            const int row = warp + r * NW;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int cc = lane + 32 * q;
+                M[r][q] = row < nr && cc < m ? __ldcg(A + (size_t)(r0 + row) * m + cc) : make_double2(0.0, 0.0);
+            }
+        }
+    }
+    __device__ void dot(const double2* v, double2 (&acc)[RW]) const {   // per lane
+#pragma unroll
+        for (int r = 0; r < RW; ++r) acc[r] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int cc = lane + 32 * q;
+            const double2 x = cc < m ? v[cc] : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int r = 0; r < RW; ++r) acc[r] = cfma(M[r][q], x, acc[r]);
+        }
+    }
+    // Sums over the warp.  Halves of the warp take one row each (RW 2), then
+    // half of those the real and half the imaginary part, so a value is
+    // exchanged once per level: lane returns the sum of part() of row().
+    __device__ int row() const { return warp + (RW == 2 ? (lane >> 4) * NW : 0); }
+    __device__ int part() const { return (RW == 2 ? lane >> 3 : lane >> 4) & 1; }
+    __device__ bool writes() const { return (lane & (RW == 2 ? 7 : 15)) == 0 && row() < nr; }
+    __device__ double reduce(const double2 (&acc)[RW]) const {
+        static_assert(RW <= 2, "two rows at most");
+        double2 v = acc[0];
+        int o = 16;
+        if constexpr (RW == 2) {
+            const bool up = (lane & 16) != 0;
+            const double2 keep = up ? acc[1] : acc[0], give = up ? acc[0] : acc[1];
+            v.x = keep.x + __shfl_xor_sync(kFull, give.x, 16);
+            v.y = keep.y + __shfl_xor_sync(kFull, give.y, 16);
+            o = 8;
+        }
+        const bool im = (lane & o) != 0;
+        double u = (im ? v.y : v.x) + __shfl_xor_sync(kFull, im ? v.x : v.y, o);
+#pragma unroll
+        for (int q = 8; q > 0; q >>= 1)
+            if (q < o) u += __shfl_xor_sync(kFull, u, q);
+        return u;
+    }
+};
+// entry p of a vector, as its two parts
+__device__ __forceinline__ double* part_of(double2* v, size_t p, int part) { return reinterpret_cast<double*>(v + p) + part; }
+
+// Forward and backward sweep of every segment (a cluster each): X of the
+// segment's lines for right-hand side f, with E = 0 on the separators
+// (seps 0) or with their values in X (seps 1).
+//   w_b = f_b - E_b y_{b-1},  y_b = D_b^{-1} w_b,  x_b = y_b - D_b^{-1} E_{b+1} x_{b+1}
+// A product takes 3 us on the 501 x 221 guide (the 15 clusters read the
+// inverses at 3.8 TB/s); a second matrix on its way through shared memory
+// made it 3.5.
+template <int NQ, int RW, int NT>
+__global__ void __launch_bounds__(NT, 1) k_fdfd_sweep(FdfdDev P, const FdSeg* __restrict__ segs,
+                                                      const double2* __restrict__ f, double2* X, int seps) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), c = (int)cl.block_rank();
+    const FdSeg seg = segs[blockIdx.x / C];
+    const int m = P.m, t = threadIdx.x;
+    FdMv<NQ, RW, NT> mv;
+    mv.m = m;
+    mv.R = (m + C - 1) / C;
+    mv.r0 = c * mv.R;
+    mv.nr = max(0, min(m, mv.r0 + mv.R) - mv.r0);
+    mv.lane = t & 31;
+    mv.warp = t >> 5;
+    __shared__ double2 s_full[2][kFdMaxM];   // the vector multiplied, by step parity
+    __shared__ double2 s_y[32];              // the own entries of the last product
+    const int d = seg.dir, first = d > 0 ? seg.a : seg.a + seg.n - 1;
+    // couplings of line b to the one before (prev) and after it, in the order of elimination
+    auto e_prev = [&](int b) { return P.eb + (size_t)(d > 0 ? b : b + 1) * m; };
+    auto e_next = [&](int b) { return P.eb + (size_t)(d > 0 ? b + 1 : b) * m; };
+    // thread t pushes entry t % nr of the vector to CTA t / nr
+    const int npush = mv.nr * C;
+    int par = 0;
+    const double2 zero = make_double2(0.0, 0.0);
+    constexpr int NPU = ((NQ > 8 ? 24 * 16 : 32 * 8) + NT - 1) / NT;   // pushes per thread at most
+    // separators next to the segment (seps)
+    const bool sp0 = seps && seg.a > 0, sp1 = seps && seg.a + seg.n < P.nb;
+
+    // the entry this thread pushes, and what forms it: f and the coupling are
+    // loaded a step ahead
+    static_assert(NPU == 1, "one entry per thread");
+    const bool pushes = t < npush;
+    const int c2 = pushes ? t / mv.nr : 0, prow = pushes ? t - c2 * mv.nr : 0, pp = mv.r0 + prow;
+    double2* const dst[2] = {cl.map_shared_rank(&s_full[0][0], c2) + pp, cl.map_shared_rank(&s_full[1][0], c2) + pp};
+    double2 fv = zero, ev = zero;
+    auto ahead_fwd = [&](int i) {   // step i of the forward sweep
+        if (!pushes || i >= seg.n) return;
+        const int b = first + d * i;
+        fv = __ldg(f + (size_t)b * m + pp);
+        if (i > 0) ev = __ldg(e_prev(b) + pp);
+        if (sp0 && b == seg.a) fv = cfms(P.eb[(size_t)b * m + pp], X[(size_t)(b - 1) * m + pp], fv);
+        if (sp1 && b == seg.a + seg.n - 1) fv = cfms(P.eb[(size_t)(b + 1) * m + pp], X[(size_t)(b + 1) * m + pp], fv);
+    };
+    auto ahead_back = [&](int i) {
+        if (pushes && i >= 0) ev = __ldg(e_next(first + d * i) + pp);
+    };
+    mv.load(P.inv + (size_t)first * m * m);
+    ahead_fwd(0);
+    // ---- forward
+    for (int i = 0; i < seg.n; ++i) {
+        const int b = first + d * i;
+        if (pushes) *dst[par] = i > 0 ? cfms(ev, s_y[prow], fv) : fv;
+        if (i + 1 < seg.n) ahead_fwd(i + 1);
+        else ahead_back(seg.n - 2);
+        cl.sync();
+        double2 acc[RW];
+        mv.dot(s_full[par], acc);
+        // the next matrix: the next line's, or (backward) the last line but one's
+        if (i + 1 < seg.n) mv.load(P.inv + (size_t)(b + d) * m * m);
+        else if (seg.n > 1) mv.load(P.inv + (size_t)(b - d) * m * m);
+        const double y = mv.reduce(acc);
+        if (mv.writes()) {
+            *part_of(s_y, mv.row(), mv.part()) = y;
+            *part_of(X, (size_t)b * m + mv.r0 + mv.row(), mv.part()) = y;
         }
         __syncthreads();
-        for (int b = nb - 2; b >= 0; --b, ++g) {
-            const int par = (int)(g & 1);
-            for (int q = t; q < nr; q += kSolveThreads) {
-                const int p = r0 + q;
-                const size_t o = (size_t)b * m + p;
-                s_pub[par][p] = cmul(P.bp[o], x[o + m]);
+        par ^= 1;
+    }
+    // ---- backward (s_y: x of the last line)
+    for (int i = seg.n - 2; i >= 0; --i) {
+        const int b = first + d * i;
+        if (pushes) *dst[par] = cmul(ev, s_y[prow]);
+        ahead_back(i - 1);
+        const double y = mv.writes() ? *part_of(X, (size_t)b * m + mv.r0 + mv.row(), mv.part()) : 0.0;
+        cl.sync();
+        double2 acc[RW];
+        mv.dot(s_full[par], acc);
+        if (i > 0) mv.load(P.inv + (size_t)(b - d) * m * m);
+        const double x = y - mv.reduce(acc);
+        if (mv.writes()) {
+            *part_of(s_y, mv.row(), mv.part()) = x;
+            *part_of(X, (size_t)b * m + mv.r0 + mv.row(), mv.part()) = x;
+        }
+        __syncthreads();
+        par ^= 1;
+    }
+    cl.sync();   // no CTA leaves while another may still write its shared memory
+}
+
+// The separators' sweeps, cluster 0 from the first one and cluster 1 from the
+// last one to the middle: phase 0 forward,
+//   z_j = r_j - Y z of the one before,  V_j = Inv_j z_j,
+// phase 1 the middle one (both clusters) and back, x_j = V_j - Y_j.' x_next.
+// r_j = f_j - E x of the lines beside it (the segments' first sweeps).
+struct FdRed {
+    int J, mid;
+    const int* line;                 // [J]
+    const double2 *Y, *YT;           // [J][m][m]: z of the next separator towards mid -= Y_j z_j
+    double2 *V, *Z;                  // [J][m], [2][m]: what reaches the middle one from each side
+};
+template <int NQ, int RW, int NT>
+__global__ void __launch_bounds__(NT, 1) k_fdfd_red(FdfdDev P, FdRed D, const double2* __restrict__ f, double2* X,
+                                                    int phase) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), c = (int)cl.block_rank(), side = (int)(blockIdx.x / C);
+    const int m = P.m, t = threadIdx.x;
+    FdMv<NQ, RW, NT> mv;
+    mv.m = m;
+    mv.R = (m + C - 1) / C;
+    mv.r0 = c * mv.R;
+    mv.nr = max(0, min(m, mv.r0 + mv.R) - mv.r0);
+    mv.lane = t & 31;
+    mv.warp = t >> 5;
+    __shared__ double2 s_full[2][kFdMaxM];
+    __shared__ double2 s_y[32];
+    const int npush = mv.nr * C;
+    int par = 0;
+    constexpr int NPU = ((NQ > 8 ? 24 * 16 : 32 * 8) + NT - 1) / NT;
+    const int d = side == 0 ? 1 : -1, j0 = side == 0 ? 0 : D.J - 1;
+    const int n = side == 0 ? D.mid : D.J - 1 - D.mid;   // separators before the middle one
+    auto rhs = [&](int j, int p) {
+        const int b = D.line[j];
+        double2 r = f[(size_t)b * m + p];
+        r = cfms(P.eb[(size_t)b * m + p], X[(size_t)(b - 1) * m + p], r);
+        return cfms(P.eb[(size_t)(b + 1) * m + p], X[(size_t)(b + 1) * m + p], r);
+    };
+    // the vector of a product, entry by entry
+    auto push = [&](auto&& value) {
+#pragma unroll
+        for (int u = 0; u < NPU; ++u) {
+            const int q = t + u * NT;
+            if (q >= npush) break;
+            const int c2 = q / mv.nr, row = q - c2 * mv.nr;
+            cl.map_shared_rank(&s_full[par][0], c2)[mv.r0 + row] = value(row, mv.r0 + row);
+        }
+        cl.sync();
+    };
+    double2 acc[RW];
+    if (phase == 0) {
+        if (n > 0) mv.load(D.Y + (size_t)j0 * m * m);
+        for (int i = 0; i < n; ++i) {
+            const int j = j0 + d * i;
+            push([&](int row, int p) {
+                const double2 r = rhs(j, p);
+                return i > 0 ? csub(r, s_y[row]) : r;
+            });
+            mv.dot(s_full[par], acc);
+            mv.load(P.inv + (size_t)D.line[j] * m * m);
+            const double y = mv.reduce(acc);   // (s_y was read before the push's cluster barrier)
+            if (mv.writes()) {
+                *part_of(s_y, mv.row(), mv.part()) = y;
+                if (i + 1 == n) *part_of(D.Z, (size_t)side * m + mv.r0 + mv.row(), mv.part()) = y;
             }
-            cl.sync();
-            for (int jj = t; jj < m; jj += kSolveThreads) s_full[jj] = cl.map_shared_rank(&s_pub[par][0], jj / R)[jj];
+            mv.dot(s_full[par], acc);
+            if (i + 1 < n) mv.load(D.Y + (size_t)(j + d) * m * m);
+            const double v = mv.reduce(acc);
+            if (mv.writes()) *part_of(D.V, (size_t)j * m + mv.r0 + mv.row(), mv.part()) = v;
             __syncthreads();
-            gemv_rows(b, Y, x);
-            __syncthreads();
+            par ^= 1;
         }
     } else {
-        // partial sums of D_b^{-T} u over the owned rows, for every column
-        auto partial = [&](int b, int par) {
-            const double2* Ib = P.inv + (size_t)b * m * m;
-            for (int jj = t; jj < m; jj += kSolveThreads) {
-                double2 acc = make_double2(0.0, 0.0);
-                for (int q = 0; q < nr; ++q) acc = cadd(acc, cmul(Ib[(size_t)(r0 + q) * m + jj], s_u[q]));
-                s_pub[par][jj] = acc;
-            }
-        };
-        auto reduce_own = [&](int par, int q) {
-            double2 s = make_double2(0.0, 0.0);
-            for (int c2 = 0; c2 < C; ++c2) s = cadd(s, cl.map_shared_rank(&s_pub[par][0], c2)[r0 + q]);
-            return s;
-        };
-        for (int b = 0; b < nb; ++b, ++g) {
-            const int par = (int)(g & 1);
-            for (int q = t; q < nr; q += kSolveThreads) {
-                const size_t o = (size_t)b * m + r0 + q;
-                double2 u = rhs[o];
-                if (b > 0) u = csub(u, cmul(P.bp[o - m], Y[o - m]));
-                s_u[q] = u;
-            }
-            __syncthreads();
-            partial(b, par);
-            cl.sync();
-            for (int q = t; q < nr; q += kSolveThreads) Y[(size_t)b * m + r0 + q] = reduce_own(par, q);
-            __syncthreads();
-        }
-        for (int q = t; q < nr; q += kSolveThreads) {
-            const size_t o = (size_t)(nb - 1) * m + r0 + q;
-            x[o] = Y[o];
+        mv.load(P.inv + (size_t)D.line[D.mid] * m * m);
+        push([&](int row, int p) {
+            (void)row;
+            double2 r = rhs(D.mid, p);
+            if (D.mid > 0) r = csub(r, D.Z[p]);
+            if (D.mid < D.J - 1) r = csub(r, D.Z[m + p]);
+            return r;
+        });
+        mv.dot(s_full[par], acc);
+        if (n > 0) mv.load(D.YT + (size_t)(D.mid - d) * m * m);
+        const double xm = mv.reduce(acc);
+        if (mv.writes()) {
+            *part_of(s_y, mv.row(), mv.part()) = xm;
+            if (side == 0) *part_of(X, (size_t)D.line[D.mid] * m + mv.r0 + mv.row(), mv.part()) = xm;
         }
         __syncthreads();
-        for (int b = nb - 1; b >= 1; --b, ++g) {
-            const int par = (int)(g & 1);
-            for (int q = t; q < nr; q += kSolveThreads) {
-                const size_t o = (size_t)b * m + r0 + q;
-                s_u[q] = cmul(P.bm[o], x[o]);
+        par ^= 1;
+        for (int i = n - 1; i >= 0; --i) {
+            const int j = j0 + d * i;
+            push([&](int row, int) { return s_y[row]; });
+            mv.dot(s_full[par], acc);
+            if (i > 0) mv.load(D.YT + (size_t)(j - d) * m * m);
+            const double v = mv.writes() ? *part_of(D.V, (size_t)j * m + mv.r0 + mv.row(), mv.part()) : 0.0;
+            const double x = v - mv.reduce(acc);
+            if (mv.writes()) {
+                *part_of(s_y, mv.row(), mv.part()) = x;
+                *part_of(X, (size_t)D.line[j] * m + mv.r0 + mv.row(), mv.part()) = x;
             }
             __syncthreads();
-            partial(b - 1, par);
-            cl.sync();
-            for (int q = t; q < nr; q += kSolveThreads) {
-                const size_t o = (size_t)(b - 1) * m + r0 + q;
-                x[o] = csub(Y[o], reduce_own(par, q));
-            }
-            __syncthreads();
+            par ^= 1;
         }
     }
-    cl.sync();   // no CTA leaves while another may still read its shared memory
+    cl.sync();   // no CTA leaves while another may still write its shared memory
 }
 
-// Factor kernel shape for block size m: CTAs of the cluster, rows per CTA
-// at most (RM), thread groups per column (TPC); threads TPC x m rounded up
-// to a warp.  m <= 128: 8 CTAs, 4 groups of 4 rows; m <= 256: 16 CTAs, 4
-// groups of 4 rows; m <= 384: 16 CTAs, one group of 24 rows.
-int fd_shape(int m, int* C, int* RM) {
-    static const int kC[3] = {8, 16, 16}, kR[3] = {16, 16, 24};
-    for (int q = 0; q < 3; ++q)
-        if (kC[q] * kR[q] >= m) {
+// The caller's vector (i + nx k) and the block layout (b m + p), with the
+// scaling by s = s_x(i) s_z(k): f = -s J (mode 0) or g (mode 1); E = x or s x.
+struct FdMap {
+    int nx, nz, along_x;
+    const double2 *sx, *sz;
+    __device__ size_t at(int i, int k) const { return along_x ? (size_t)i * nz + k : (size_t)k * nx + i; }
+};
+__global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __restrict__ f, int mode) {
+    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
+         g += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
+        double2 x = v[g];
+        if (mode == 0) {
+            x = cmul(cmul(mp.sx[i], mp.sz[k]), x);
+            x = make_double2(-x.x, -x.y);
+        }
+        f[mp.at(i, k)] = x;
+    }
+}
+__global__ void k_fd_out(FdMap mp, const double2* __restrict__ x, double2* __restrict__ v, int mode) {
+    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
+         g += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
+        const double2 y = x[mp.at(i, k)];
+        v[g] = mode == 0 ? y : cmul(cmul(mp.sx[i], mp.sz[k]), y);
+    }
+}
+// r = f - M x and the largest |r|^2, |x|^2 and |f|^2 (bits of non-negative
+// doubles order as integers); add: x += dx first
+__global__ void k_fd_residual(FdfdDev P, const double2* __restrict__ f, const double2* __restrict__ x,
+                              double2* __restrict__ r, unsigned long long* mx) {
+    const size_t N = (size_t)P.nb * P.m;
+    double v[3] = {0.0, 0.0, 0.0};
+    bool nan = false;
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < N; o += (size_t)gridDim.x * blockDim.x) {
+        const int b = (int)(o / P.m), p = (int)(o - (size_t)b * P.m);
+        const double2 xo = x[o], fo = f[o];
+        double2 s = cfms(P.diag[o], xo, fo);
+        if (p > 0) s = cfms(P.wc[o], x[o - 1], s);
+        if (p + 1 < P.m) s = cfms(P.wc[o + 1], x[o + 1], s);
+        if (b > 0) s = cfms(P.eb[o], x[o - P.m], s);
+        if (b + 1 < P.nb) s = cfms(P.eb[o + P.m], x[o + P.m], s);
+        r[o] = s;
+        const double a[3] = {cabs2(s), cabs2(xo), cabs2(fo)};
+        for (int q = 0; q < 3; ++q) {
+            nan = nan || !(a[q] >= 0.0);
+            v[q] = fmax(v[q], a[q]);
+        }
+    }
+    if (nan) v[0] = CUDART_INF;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[q] = fmax(v[q], __shfl_xor_sync(kFull, v[q], o));
+        if ((threadIdx.x & 31) == 0) atomicMax(mx + q, (unsigned long long)__double_as_longlong(v[q]));
+    }
+}
+__global__ void k_fd_add(double2* __restrict__ x, const double2* __restrict__ dx, size_t n) {
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x)
+        x[o] = cadd(x[o], dx[o]);
+}
+// the right-hand side a factorisation is tried on: of magnitude one everywhere, no pattern
+__global__ void k_fd_probe(double2* f, size_t n) {
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+        unsigned h = (unsigned)o * 2654435761u;
+        h ^= h >> 15;
+        h *= 2246822519u;
+        h ^= h >> 13;
+        f[o] = make_double2((double)(h & 0xffffu) / 32768.0 - 1.0, (double)(h >> 16) / 32768.0 - 1.0);
+    }
+}
+
+// Shape for block size m: CTAs of a cluster (rows per CTA: at most 32, 24 for
+// the 16 of a non-portable cluster).
+int fd_shape(int m, int* C) {
+    static const int kC[4] = {2, 4, 8, 16}, kM[4] = {64, 128, 256, kFdMaxM};
+    for (int q = 0; q < 4; ++q)
+        if (m <= kM[q]) {
             *C = kC[q];
-            *RM = kR[q];
             return ORF_OK;
         }
     set_error("fdfd2D: the shorter grid axis has %d points, above the %d this solver takes", m, kFdMaxM);
@@ -678,17 +796,18 @@ int fd_shape(int m, int* C, int* RM) {
 }
 
 template <class K, class... Args>
-cudaError_t launch_cluster(K kern, int C, int threads, size_t smem, cudaStream_t s, Args... args) {
+cudaError_t launch_cluster(K kern, int clusters, int C, int threads, size_t smem, cudaStream_t s, int* most,
+                           Args... args) {
     if (C > 8) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    if (smem > 48 * 1024) {
+    if (smem > 32 * 1024) {   // (the kernels' static arrays count too)
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)C, 1, 1);
+    cfg.gridDim = dim3((unsigned)(C * clusters), 1, 1);
     cfg.blockDim = dim3((unsigned)threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -699,7 +818,47 @@ cudaError_t launch_cluster(K kern, int C, int threads, size_t smem, cudaStream_t
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    if (most) return cudaOccupancyMaxActiveClusters(most, kern, &cfg);   // resident at once; no launch
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// the factor kernel of block size m (most: only ask how many clusters fit)
+cudaError_t launch_factor(const FdfdDev& P, int C, const FdSeg* segs, int n, cudaStream_t s, int* most) {
+    const int mp = (P.m + 31) / 32 * 32, R = (P.m + C - 1) / C;
+    const size_t smem = fd_factor_smem(P.m, R);
+    if (C <= 4) return launch_cluster(k_fdfd_factor<8, 4, 512>, n, C, 4 * mp, smem, s, most, P, segs);
+    if (C == 8) return launch_cluster(k_fdfd_factor<16, 2, 512>, n, C, 2 * mp, smem, s, most, P, segs);
+    return launch_cluster(k_fdfd_factor<24, 1, 384>, n, C, mp, smem, s, most, P, segs);
+}
+cudaError_t launch_sweep(const FdfdDev& P, int C, const FdSeg* segs, int n, const double2* f, double2* X, int seps,
+                         cudaStream_t s) {
+    if (C == 2) return launch_cluster(k_fdfd_sweep<2, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
+    if (C == 4) return launch_cluster(k_fdfd_sweep<4, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
+    if (C == 8) return launch_cluster(k_fdfd_sweep<8, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
+    return launch_cluster(k_fdfd_sweep<12, 2, 384>, n, C, 384, 0, s, nullptr, P, segs, f, X, seps);
+}
+cudaError_t launch_red(const FdfdDev& P, int C, const FdRed& D, const double2* f, double2* X, int phase,
+                       cudaStream_t s) {
+    if (C == 2) return launch_cluster(k_fdfd_red<2, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
+    if (C == 4) return launch_cluster(k_fdfd_red<4, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
+    if (C == 8) return launch_cluster(k_fdfd_red<8, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
+    return launch_cluster(k_fdfd_red<12, 2, 384>, 2, C, 384, 0, s, nullptr, P, D, f, X, phase);
+}
+
+// Segments for nb lines when `most` clusters run at once: the chain is
+// nb / S inversions in the segments and S / 2 at the separators (each with two
+// matrix products behind it), so as many as fit, up to about sqrt(2 nb).
+int fd_segments(int nb, int most) {
+    int best = 1;
+    double best_t = nb;
+    for (int S = 2; S <= most && nb - (S - 1) >= 4 * S; ++S) {
+        const double t = std::ceil((double)(nb - (S - 1)) / S) * (S > 2 ? 1.15 : 1.0) + 1.2 * (S / 2);
+        if (t < best_t) {
+            best_t = t;
+            best = S;
+        }
+    }
+    return best;
 }
 
 using cplx = std::complex<double>;
@@ -733,12 +892,18 @@ using namespace orf;
 
 struct orf_fdfd {
     orf_ctx* ctx = nullptr;
-    int nx = 0, nz = 0, m = 0, nb = 0, C = 8, RM = 16;
+    int nx = 0, nz = 0, m = 0, nb = 0, C = 8;
     bool along_x = true;   // blocks are lines of constant x (m = nz)
+    int S = 1;             // segments
+    double mnorm = 0.0;    // bound of the row sums of |M|
     Arena ar;
-    double2 *diag = nullptr, *wm = nullptr, *wp = nullptr, *bm = nullptr, *bp = nullptr;
-    double2 *inv = nullptr, *Y = nullptr, *vin = nullptr, *vout = nullptr, *xpan = nullptr, *xrow = nullptr;
-    int* fault = nullptr;
+    double2 *diag = nullptr, *wc = nullptr, *eb = nullptr, *sx = nullptr, *sz = nullptr;
+    double2 *inv = nullptr, *vin = nullptr, *vout = nullptr, *xrow = nullptr;
+    double2 *f = nullptr, *x = nullptr, *r = nullptr, *dx = nullptr, *Y = nullptr, *YT = nullptr, *V = nullptr,
+            *Z = nullptr;
+    unsigned long long* mx = nullptr;
+    FdSeg* segs = nullptr;
+    int *line = nullptr, *fault = nullptr;
     ~orf_fdfd() {
         if (ar.base) {
             cudaStreamSynchronize(ctx->stream);
@@ -746,10 +911,198 @@ struct orf_fdfd {
         }
         if (ctx) ctx_release(ctx);
     }
-    FdfdDev dev() const { return FdfdDev{m, nb, diag, wm, wp, bm, bp, inv, fault, xpan, xrow}; }
+    FdfdDev dev() const { return FdfdDev{m, nb, diag, wc, eb, inv, fault, xrow}; }
+    FdMap map() const { return FdMap{nx, nz, along_x ? 1 : 0, sx, sz}; }
+    size_t N() const { return (size_t)nx * nz; }
     // (i, k) of the grid <-> entry b * m + p of the block layout
     size_t at(int i, int k) const { return along_x ? (size_t)i * m + k : (size_t)k * m + i; }
+    // x of M x = f for the right-hand side in `rhs`, into `out`
+    int solve(const double2* rhs, double2* out) {
+        cudaStream_t st = ctx->stream;
+        const FdfdDev P = dev();
+        ORF_CUDA(launch_sweep(P, C, segs, S, rhs, out, 0, st));
+        if (S > 1) {
+            const FdRed D{S - 1, (S - 1) / 2, line, Y, YT, V, Z};
+            ORF_CUDA(launch_red(P, C, D, rhs, out, 0, st));
+            ORF_CUDA(launch_red(P, C, D, rhs, out, 1, st));
+            ORF_CUDA(launch_sweep(P, C, segs, S, rhs, out, 1, st));
+        }
+        return ORF_OK;
+    }
+    // r = f - M x, and its size against rounding: |r| / (|M| |x| + |f|), largest entries
+    int residual(double* eta) {
+        cudaStream_t st = ctx->stream;
+        ORF_CUDA(cudaMemsetAsync(mx, 0, 3 * sizeof *mx, st));
+        k_fd_residual<<<296, 256, 0, st>>>(dev(), f, x, r, mx);
+        ORF_CUDA(cudaGetLastError());
+        double h[3];
+        ORF_CUDA(cudaMemcpyAsync(h, mx, sizeof h, cudaMemcpyDeviceToHost, st));
+        ORF_CUDA(cudaStreamSynchronize(st));
+        const double den = mnorm * std::sqrt(h[1]) + std::sqrt(h[2]);
+        *eta = h[0] == 0.0 ? 0.0 : std::sqrt(h[0]) / den;
+        return ORF_OK;
+    }
+    int refine() {
+        ORF_TRY(solve(r, dx));
+        k_fd_add<<<296, 256, 0, ctx->stream>>>(x, dx, N());
+        ORF_CUDA(cudaGetLastError());
+        return ORF_OK;
+    }
+    int factor(int nseg, bool* singular);
 };
+
+namespace {
+// A solve with a residual above kEtaRefine takes a step of refinement: as one
+// segment the residuals are 6e-17 .. 1.3e-16 (error against an exact solve
+// 2e-14 .. 1.4e-13 on grids of 150 x 92 .. 600 x 250), as 15 segments 1e-16 ..
+// 5e-15 (up to 3e-12), and 1e-17 (2e-14 .. 9e-14) after the step.  A
+// factorisation whose trial solve has one above kEtaTrial is done again as
+// one segment.
+constexpr double kEtaRefine = 1e-16, kEtaTrial = 1e-11;
+}  // namespace
+
+// Factor the operator as nseg segments.
+int orf_fdfd::factor(int nseg, bool* singular) {
+    cudaStream_t st = ctx->stream;
+    const FdfdDev P = dev();
+    const size_t mm = (size_t)m * m;
+    S = nseg;
+    const int J = S - 1;
+    // the segments' lines: equal shares of the lines that are not separators
+    std::vector<FdSeg> hs(S);
+    std::vector<int> sep(J);
+    {
+        int a = 0;
+        for (int s = 0; s < S; ++s) {
+            const int n = (int)((int64_t)(nb - J) * (s + 1) / S - (int64_t)(nb - J) * s / S);
+            hs[s] = FdSeg{a, n, s > 0 && s == S - 1 ? -1 : 1, 0, nullptr};
+            a += n;
+            if (s < J) sep[s] = a++;
+        }
+    }
+    ORF_CUDA(cudaMemsetAsync(fault, 0, sizeof(int), st));
+    ORF_CUDA(cudaMemcpyAsync(segs, hs.data(), S * sizeof(FdSeg), cudaMemcpyHostToDevice, st));
+    ORF_CUDA(launch_factor(P, C, segs, S, st, nullptr));
+    Arena tmp;   // the separators' blocks and the corner blocks of the segments' inverses
+    struct Release {
+        Arena& a;
+        cudaStream_t s;
+        ~Release() {
+            if (a.base) {
+                cudaStreamSynchronize(s);
+                a.release();
+            }
+        }
+    } rel{tmp, st};
+    if (J > 0) {
+        ORF_CUDA(cudaMemcpyAsync(line, sep.data(), J * sizeof(int), cudaMemcpyHostToDevice, st));
+        const int nin = std::max(0, S - 2);   // segments with two separators: 1 .. S-2
+        double2 *Kd, *T, *L, *F;
+        FdGemm* d_g;
+        FdSepIn* d_sep;
+        FdSeg* d_dense;
+        int tmax = 0;
+        for (int s = 1; s <= nin; ++s) tmax = std::max(tmax, hs[s].n);
+        const int mid = J / 2;
+        // ---- the batches of matrix products, in order: the corner blocks
+        // (step t: L_t of every segment, F of step t - 1), then the separators'
+        tmp.add(&Kd, J * mm);
+        tmp.add(&T, J * mm);
+        tmp.add(&L, (size_t)std::max(1, 3 * nin) * mm);
+        tmp.add(&F, (size_t)std::max(1, nin) * mm);
+        tmp.add(&d_g, (size_t)2 * nin * (tmax + 1) + 2 * J + 1);
+        tmp.add(&d_sep, J);
+        tmp.add(&d_dense, J);
+        ORF_TRY(tmp.alloc());
+        std::vector<FdGemm> g;
+        std::vector<std::pair<int, int>> batch;   // [first, end) in g
+        auto Lp = [&](int s, int t) -> double2* {   // L_t of segment s
+            return t == 0 ? inv + (size_t)hs[s].a * mm : L + ((size_t)3 * (s - 1) + t % 3) * mm;
+        };
+        for (int t = 1; t <= tmax; ++t) {
+            const int g0 = (int)g.size();
+            for (int s = 1; s <= nin; ++s) {
+                const int n = hs[s].n;
+                const double2* e = eb + (size_t)(hs[s].a + t) * m;
+                if (t < n) g.push_back(FdGemm{inv + (size_t)(hs[s].a + t) * mm, Lp(s, t - 1), nullptr, e, Lp(s, t), 0, 0, -1.0});
+                if (t >= 2 && t - 1 < n) {
+                    double2* Fs = F + (size_t)(s - 1) * mm;
+                    g.push_back(FdGemm{Lp(s, t - 1), Lp(s, t - 2), t == 2 ? Lp(s, 0) : Fs, e - m, Fs, 1, 0, -1.0});
+                }
+            }
+            batch.push_back({g0, (int)g.size()});
+        }
+        const size_t nspike = batch.size();
+        // ---- elimination of the separators: the blocks of each step
+        std::vector<FdSepIn> si(J);
+        std::vector<FdSeg> dense;
+        std::vector<int> dense_n;
+        for (int q = 0; q < J; ++q) {
+            // segment q before the separator (its last line eliminated last),
+            // segment q + 1 after it (the last segment runs downwards)
+            const double2* first = q + 1 == S - 1 ? inv + (size_t)hs[S - 1].a * mm
+                                   : hs[q + 1].n == 1 ? inv + (size_t)hs[q + 1].a * mm : F + (size_t)q * mm;
+            si[q] = FdSepIn{sep[q], q > 0 ? 1 : 0, inv + (size_t)(sep[q] - 1) * mm, first,
+                            q > 0 ? Lp(q, hs[q].n - 1) : nullptr};
+        }
+        for (int i = 0; i <= std::max(mid, J - 1 - mid); ++i) {
+            const int lo = i, hi = J - 1 - i;
+            const bool l = lo < mid, h = hi > mid;
+            int n = 0;
+            if (l) dense.push_back(FdSeg{sep[lo], 1, 1, 0, Kd + (size_t)lo * mm}), ++n;
+            if (h) dense.push_back(FdSeg{sep[hi], 1, 1, 0, Kd + (size_t)hi * mm}), ++n;
+            if (!l && !h) {
+                dense.push_back(FdSeg{sep[mid], 1, 1, 0, Kd + (size_t)mid * mm});
+                dense_n.push_back(1);
+                break;
+            }
+            dense_n.push_back(n);
+            const int g0 = (int)g.size();
+            if (l) g.push_back(FdGemm{T + (size_t)(lo + 1) * mm, inv + (size_t)sep[lo] * mm, nullptr, nullptr, Y + (size_t)lo * mm, 0, 0, 1.0});
+            if (h) g.push_back(FdGemm{T + (size_t)hi * mm, inv + (size_t)sep[hi] * mm, nullptr, nullptr, Y + (size_t)hi * mm, 1, 0, 1.0});
+            batch.push_back({g0, (int)g.size()});
+            // (the two updates may meet in the middle block: one launch each)
+            if (l) {
+                double2* K = Kd + (size_t)(lo + 1) * mm;
+                g.push_back(FdGemm{Y + (size_t)lo * mm, T + (size_t)(lo + 1) * mm, K, nullptr, K, 0, 1, -1.0});
+                batch.push_back({(int)g.size() - 1, (int)g.size()});
+            }
+            if (h) {
+                double2* K = Kd + (size_t)(hi - 1) * mm;
+                g.push_back(FdGemm{Y + (size_t)hi * mm, T + (size_t)hi * mm, K, nullptr, K, 0, 0, -1.0});
+                batch.push_back({(int)g.size() - 1, (int)g.size()});
+            }
+        }
+        ORF_CUDA(cudaMemcpyAsync(d_g, g.data(), g.size() * sizeof(FdGemm), cudaMemcpyHostToDevice, st));
+        ORF_CUDA(cudaMemcpyAsync(d_sep, si.data(), J * sizeof(FdSepIn), cudaMemcpyHostToDevice, st));
+        ORF_CUDA(cudaMemcpyAsync(d_dense, dense.data(), dense.size() * sizeof(FdSeg), cudaMemcpyHostToDevice, st));
+        const unsigned nt = (unsigned)((m + kGT - 1) / kGT);
+        size_t bq = 0;
+        auto products = [&]() -> cudaError_t {
+            const auto [a, b] = batch[bq++];
+            if (b > a) k_fd_gemm<<<dim3(nt, nt, (unsigned)(b - a)), kGN, 0, st>>>(d_g + a, m);
+            return cudaGetLastError();
+        };
+        while (bq < nspike) ORF_CUDA(products());
+        k_fd_assemble<<<dim3((unsigned)m, (unsigned)J), 128, 0, st>>>(P, d_sep, Kd, T);
+        ORF_CUDA(cudaGetLastError());
+        int dq = 0;
+        for (size_t i = 0; i < dense_n.size(); ++i) {
+            ORF_CUDA(launch_factor(P, C, d_dense + dq, dense_n[i], st, nullptr));
+            dq += dense_n[i];
+            if (i + 1 < dense_n.size())
+                for (int q = 0; q < 1 + dense_n[i]; ++q) ORF_CUDA(products());
+        }
+        const unsigned tt = (unsigned)((m + 15) / 16);
+        k_fd_transpose<<<dim3(tt, tt, (unsigned)J), dim3(16, 16), 0, st>>>(Y, YT, m);
+        ORF_CUDA(cudaGetLastError());
+    }
+    int flt = 0;
+    ORF_CUDA(cudaMemcpyAsync(&flt, fault, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ORF_CUDA(cudaStreamSynchronize(st));
+    *singular = flt != 0;
+    return ORF_OK;
+}
 
 extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdfd** out) {
     if (!out) {
@@ -781,69 +1134,106 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
     F->along_x = nz <= nx;
     F->m = F->along_x ? nz : nx;
     F->nb = F->along_x ? nx : nz;
-    ORF_TRY(fd_shape(F->m, &F->C, &F->RM));
+    ORF_TRY(fd_shape(F->m, &F->C));
     const int m = F->m, nb = F->nb;
-    const size_t N = (size_t)nx * nz;
+    const size_t N = F->N();
 
-    // ---- operator coefficients, rows scaled as in A E = -J
+    // ---- M = diag(s_x s_z) A, symmetric
     const double d = pr->dx, k0 = 2.0 * kPi / pr->lambda0, R = pr->pml_reflection;
     const auto sxi = fd_stretch(nx, pr->npml_x, d, k0, R, false), sxh = fd_stretch(nx, pr->npml_x, d, k0, R, true);
     const auto szi = fd_stretch(nz, pr->npml_z, d, k0, R, false), szh = fd_stretch(nz, pr->npml_z, d, k0, R, true);
-    std::vector<double2> hd(N), hwm(N), hwp(N), hbm(N), hbp(N);
+    std::vector<double2> hd(N), hw(N), he(N);
     const double h2 = 1.0 / (d * d);
     auto d2 = [](cplx v) { return make_double2(v.real(), v.imag()); };
+    std::vector<cplx> rxh(nx + 1), rzh(nz + 1);
+    for (int i = 0; i <= nx; ++i) rxh[i] = h2 / sxh[i];
+    for (int k = 0; k <= nz; ++k) rzh[k] = h2 / szh[k];
     for (int k = 0; k < nz; ++k)
         for (int i = 0; i < nx; ++i) {
-            const cplx cxm = h2 / (sxi[i] * sxh[i]), cxp = h2 / (sxi[i] * sxh[i + 1]);
-            const cplx czm = h2 / (szi[k] * szh[k]), czp = h2 / (szi[k] * szh[k + 1]);
+            const cplx cx = szi[k] * rxh[i], cz = sxi[i] * rzh[k];   // to (i-1, k), to (i, k-1)
             const size_t g = (size_t)i + (size_t)nx * k;
             const cplx eps(pr->eps[2 * g], pr->eps[2 * g + 1]);
-            const cplx dg = -(cxm + cxp + czm + czp) + k0 * k0 * eps;
+            const cplx ax = szi[k] * (rxh[i] + rxh[i + 1]), az = sxi[i] * (rzh[k] + rzh[k + 1]);
+            const cplx dg = -(ax + az) + k0 * k0 * eps * sxi[i] * szi[k];
             const size_t o = F->at(i, k);
             hd[o] = d2(dg);
-            hwm[o] = d2(F->along_x ? czm : cxm);
-            hwp[o] = d2(F->along_x ? czp : cxp);
-            hbm[o] = d2(F->along_x ? cxm : czm);
-            hbp[o] = d2(F->along_x ? cxp : czp);
+            hw[o] = d2(F->along_x ? cz : cx);
+            he[o] = d2(F->along_x ? cx : cz);
+            F->mnorm = std::max(F->mnorm, std::abs(dg) + std::abs(ax) + std::abs(az));
         }
 
     F->ctx = ctx;
     ctx_retain(ctx);
-    Arena& ar = F->ar;
-    ar.add(&F->diag, N);
-    ar.add(&F->wm, N);
-    ar.add(&F->wp, N);
-    ar.add(&F->bm, N);
-    ar.add(&F->bp, N);
-    ar.add(&F->inv, (size_t)nb * m * m);
-    ar.add(&F->Y, N);
-    ar.add(&F->vin, N);
-    ar.add(&F->vout, N);
-    ar.add(&F->fault, 1);
-    ar.add(&F->xpan, (size_t)m * 8);
-    ar.add(&F->xrow, (size_t)8 * m);
-    ORF_TRY(ar.alloc());
     cudaStream_t st = ctx->stream;
+    int most = 1;
+    {
+        FdfdDev P{};
+        P.m = m;
+        P.nb = nb;
+        ORF_CUDA(launch_factor(P, F->C, nullptr, 1, st, &most));
+    }
+    int S = fd_segments(nb, most);
+    Arena& ar = F->ar;
+    auto carve = [&]() {
+        const int J = S - 1;
+        ar = Arena{};
+        ar.add(&F->diag, N);
+        ar.add(&F->wc, N + 1);
+        ar.add(&F->eb, N + m);   // (read one line past the last, unused)
+        ar.add(&F->sx, nx);
+        ar.add(&F->sz, nz);
+        ar.add(&F->inv, (size_t)nb * m * m);
+        ar.add(&F->vin, N);
+        ar.add(&F->vout, N);
+        ar.add(&F->f, N);
+        ar.add(&F->x, N);
+        ar.add(&F->r, N);
+        ar.add(&F->dx, N);
+        ar.add(&F->Y, (size_t)J * m * m);
+        ar.add(&F->YT, (size_t)J * m * m);
+        ar.add(&F->V, (size_t)J * m);
+        ar.add(&F->Z, (size_t)2 * m);
+        ar.add(&F->mx, 3);
+        ar.add(&F->segs, S);
+        ar.add(&F->line, J);
+        ar.add(&F->fault, 1);
+        ar.add(&F->xrow, (size_t)S * kPanel * m);
+        return ar.alloc();
+    };
+    int rc = carve();
+    if (rc != ORF_OK && S > 1) {   // one segment needs no memory for separators
+        S = 1;
+        rc = carve();
+    }
+    ORF_TRY(rc);
     ORF_CUDA(cudaMemcpyAsync(F->diag, hd.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    ORF_CUDA(cudaMemcpyAsync(F->wm, hwm.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    ORF_CUDA(cudaMemcpyAsync(F->wp, hwp.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    ORF_CUDA(cudaMemcpyAsync(F->bm, hbm.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    ORF_CUDA(cudaMemcpyAsync(F->bp, hbp.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    ORF_CUDA(cudaMemsetAsync(F->fault, 0, sizeof(int), st));
-    add_h2d(ctx, (int64_t)(5 * N * sizeof(double2)));
-    const int mp = (m + 31) / 32 * 32;
-    const FdfdDev P = F->dev();
-    cudaError_t e;
-    const size_t fsm = 0;
-    const size_t psm = fd_panel_smem(m);
-    if (F->RM == 16 && mp <= 128) e = launch_cluster(k_fdfd_factor_panel<4, 4, 512>, F->C, 4 * mp, psm, st, P);
-    else if (F->RM == 16) e = launch_cluster(k_fdfd_factor_panel<8, 2, 512>, F->C, 2 * mp, psm, st, P);
-    else e = launch_cluster(k_fdfd_factor<24, 1, 384>, F->C, mp, fsm, st, P);
-    ORF_CUDA(e);
-    int fault = 0;
-    ORF_CUDA(cudaMemcpyAsync(&fault, F->fault, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ORF_CUDA(cudaStreamSynchronize(st));
-    if (fault) {
+    ORF_CUDA(cudaMemcpyAsync(F->wc, hw.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
+    ORF_CUDA(cudaMemcpyAsync(F->eb, he.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
+    std::vector<double2> hx(nx), hz(nz);
+    for (int i = 0; i < nx; ++i) hx[i] = d2(sxi[i]);
+    for (int k = 0; k < nz; ++k) hz[k] = d2(szi[k]);
+    ORF_CUDA(cudaMemcpyAsync(F->sx, hx.data(), nx * sizeof(double2), cudaMemcpyHostToDevice, st));
+    ORF_CUDA(cudaMemcpyAsync(F->sz, hz.data(), nz * sizeof(double2), cudaMemcpyHostToDevice, st));
+    add_h2d(ctx, (int64_t)((3 * N + nx + nz) * sizeof(double2)));
+    bool singular = false;
+    rc = F->factor(S, &singular);
+    if (rc != ORF_OK && S > 1) {   // (no memory for the separators' blocks)
+        S = 1;
+        rc = F->factor(S, &singular);
+    }
+    ORF_TRY(rc);
+    if (S > 1) {
+        // a segment that is nearly singular by itself shows in a trial solve
+        double eta = 0.0;
+        if (!singular) {
+            k_fd_probe<<<296, 256, 0, st>>>(F->f, N);
+            ORF_CUDA(cudaGetLastError());
+            ORF_TRY(F->solve(F->f, F->x));
+            ORF_TRY(F->residual(&eta));
+        }
+        if (singular || !(eta <= kEtaTrial)) ORF_TRY(F->factor(1, &singular));
+    }
+    if (singular) {
         set_error("fdfd2D: the operator is singular (a zero pivot in the block elimination)");
         return ORF_EINVAL;
     }
@@ -857,28 +1247,33 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
         return ORF_EINVAL;
     }
     ORF_ON_DEVICE(F->ctx->device);
-    const size_t N = (size_t)F->nx * F->nz;
-    std::vector<double2> h(N);
-    for (int k = 0; k < F->nz; ++k)
-        for (int i = 0; i < F->nx; ++i) {
-            const size_t g = (size_t)i + (size_t)F->nx * k;
-            h[F->at(i, k)] = make_double2(rhs[2 * g], rhs[2 * g + 1]);
-        }
+    const size_t bytes = F->N() * sizeof(double2);
+    const int mode = transpose ? 1 : 0;
     cudaStream_t st = F->ctx->stream;
-    ORF_CUDA(cudaMemcpyAsync(F->vin, h.data(), N * sizeof(double2), cudaMemcpyHostToDevice, st));
-    add_h2d(F->ctx, (int64_t)(N * sizeof(double2)));
-    ORF_CUDA(launch_cluster(k_fdfd_solve, F->C, kSolveThreads, 0, st, F->dev(), (const double2*)F->vin, F->vout, F->Y,
-                            transpose ? 1 : 0));
-    ORF_CUDA(cudaMemcpyAsync(h.data(), F->vout, N * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    ORF_CUDA(cudaStreamSynchronize(st));
-    add_d2h(F->ctx, (int64_t)(N * sizeof(double2)));
-    for (int k = 0; k < F->nz; ++k)
-        for (int i = 0; i < F->nx; ++i) {
-            const size_t g = (size_t)i + (size_t)F->nx * k;
-            const double2 v = h[F->at(i, k)];
-            x[2 * g] = v.x;
-            x[2 * g + 1] = v.y;
+    void* stage = nullptr;
+    ORF_TRY(pinned_stage_acquire(&stage));
+    struct Release {
+        void* s;
+        cudaStream_t st;
+        ~Release() {
+            cudaStreamSynchronize(st);   // (after an error a copy may still be on its way)
+            pinned_stage_release(s);
         }
+    } rel{stage, st};
+    ORF_TRY(copy_h2d_staged(F->vin, rhs, bytes, stage, st));
+    add_h2d(F->ctx, (int64_t)bytes);
+    k_fd_in<<<296, 256, 0, st>>>(F->map(), F->vin, F->f, mode);
+    ORF_CUDA(cudaGetLastError());
+    ORF_TRY(F->solve(F->f, F->x));
+    if (F->S > 1) {
+        double eta = 0.0;
+        ORF_TRY(F->residual(&eta));
+        if (eta > kEtaRefine) ORF_TRY(F->refine());
+    }
+    k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode);
+    ORF_CUDA(cudaGetLastError());
+    ORF_TRY(copy_d2h_staged(x, F->vout, bytes, stage, st));
+    add_d2h(F->ctx, (int64_t)bytes);
     return ORF_OK;
 }
 

@@ -258,6 +258,18 @@ int copy_d2h_staged(void* dst, const void* src, size_t bytes, void* stage, cudaS
     return ORF_OK;
 }
 
+int copy_h2d_staged(void* dst, const void* src, size_t bytes, void* stage, cudaStream_t st) {
+    char* d = static_cast<char*>(dst);
+    const char* s = static_cast<const char*>(src);
+    for (size_t off = 0; off < bytes; off += kStageBytes) {
+        const size_t n = std::min(kStageBytes, bytes - off);
+        if (off > 0) ORF_CUDA(cudaStreamSynchronize(st));   // the chunk before has left the buffer
+        std::memcpy(stage, s + off, n);
+        ORF_CUDA(cudaMemcpyAsync(d + off, stage, n, cudaMemcpyHostToDevice, st));
+    }
+    return ORF_OK;
+}
+
 namespace {
 // one table: distinct values in first-occurrence order, with the last value
 // remembered (neighbouring cells mostly share a material)

@@ -143,6 +143,9 @@ void pinned_stage_release(void* buf);
 // Device-to-host copy of `bytes` from `src` into the pageable `dst` through
 // the staging buffer `stage`, on stream st (synchronises st).
 int copy_d2h_staged(void* dst, const void* src, size_t bytes, void* stage, cudaStream_t st);
+// The other way: bytes from host src to device dst through `stage`, which
+// stays in use until st has reached this point.
+int copy_h2d_staged(void* dst, const void* src, size_t bytes, void* stage, cudaStream_t st);
 
 // Exact dense index of the distinct values of a list of rows, in the order
 // of their first occurrence when the rows are scanned in order: dst[i] of a

@@ -65,3 +65,43 @@ def test_fdfd_rejects_a_block_above_the_limit():
     with pytest.raises(orf.OrfError) as ei:
         orf.fdfd2D(x, x, np.ones((400, 400)), 1.55, np.zeros((400, 400)))
     assert ei.value.identifier == "orf:tooLarge"
+
+
+@pytest.mark.parametrize("nx,nz", [(3, 5), (9, 3), (64, 90), (80, 65), (128, 140), (131, 129), (256, 260), (258, 257),
+                                   (384, 386)])
+def test_fdfd_block_shapes(nx, nz):
+    """Blocks at the edges of the cluster shapes (up to 64, 128, 256 and 384
+    points), grids of one segment and of many, and the trailing rows and
+    panels that a cluster's CTAs share unevenly."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(nx, nz, 3 * nx + nz, True, npml=(min(8, (nx - 1) // 2),
+                                                                                        min(6, (nz - 1) // 2)))
+    J[nx // 3, nz // 4:3 * nz // 4 + 1] = 1.0 + 0.3j   # (a line current on the smallest grids too)
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    r = oracle_fdfd2D(x, z, eps, lam, J, Npml=npml)
+    assert rel(o.E, r.E) <= TOL
+    assert rel(o.adjoint(g), r.adjoint(g)) <= TOL
+    o.close()
+
+
+def test_fdfd_segment_in_resonance():
+    """A closed lossless cavity with five segments of five lines that, cut off
+    by themselves, are exactly in resonance (k0^2 eps is an eigenvalue of the
+    5 x 6-point Laplacian: condition number 1e17); the first and the last five
+    lines hold other materials, so neither the whole grid (1.9e2) nor what the
+    elimination from the first line meets (2.7e3) is.  The factorisation has
+    to notice and go on as one segment.  41 lines are cut into seven segments
+    of five and six separators."""
+    nx, nz, d, lam = 41, 6, 0.03, 1.3
+    k0 = 2 * np.pi / lam
+    ev = 4 / d ** 2 * (np.sin(np.pi / (2 * 6)) ** 2 + np.sin(np.pi / (2 * 7)) ** 2)
+    eps = np.full((nx, nz), ev / k0 ** 2)
+    eps[:5] *= 1.3
+    eps[36:] *= 1.5
+    rng = np.random.default_rng(5)
+    J = rng.standard_normal((nx, nz)) + 1j * rng.standard_normal((nx, nz))
+    x, z = np.arange(nx) * d, np.arange(nz) * d
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=(0, 0))
+    r = oracle_fdfd2D(x, z, eps, lam, J, Npml=(0, 0))
+    assert rel(o.E, r.E) <= TOL
+    assert rel(o.adjoint(J), r.adjoint(J)) <= TOL
+    o.close()
