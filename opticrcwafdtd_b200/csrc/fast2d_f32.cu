@@ -55,10 +55,10 @@ int occv(bool te, bool idx16) {
 
 cudaError_t launch_fast2d_f32(bool te, bool idx16, bool pml, int variant, const FastTile2D* tiles, int ntiles,
                               int off, int nsub, int par, int we, int grid, cudaStream_t s) {
-    if (pml) return dispatch<true, 8, 2, 5>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
+    if (pml) return dispatch<true, 4, 2, 10>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
     switch (variant) {
-        case 1: return dispatch<false, 16, 4, 4>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
-        case 2: return dispatch<false, 8, 4, 4>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
+        case 1: return dispatch<false, 8, 4, 8>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
+        case 2: return dispatch<false, 4, 4, 8>(te, idx16, tiles, ntiles, off, nsub, par, we, grid, s);
     }
     return cudaErrorInvalidValue;
 }
@@ -81,10 +81,10 @@ int fast2d_violations_f32(unsigned long long* n, int reset) {
 }
 
 int occ_fast2d_f32(bool te, bool idx16, bool pml, int variant) {
-    if (pml) return occv<true, 8, 2, 5>(te, idx16);
+    if (pml) return occv<true, 4, 2, 10>(te, idx16);
     switch (variant) {
-        case 1: return occv<false, 16, 4, 4>(te, idx16);
-        case 2: return occv<false, 8, 4, 4>(te, idx16);
+        case 1: return occv<false, 8, 4, 8>(te, idx16);
+        case 2: return occv<false, 4, 4, 8>(te, idx16);
     }
     return 0;
 }

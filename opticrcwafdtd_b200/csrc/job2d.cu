@@ -74,7 +74,10 @@ int plan2d(const orf_sim2d* s, const orf_tuning& tuning, Plan2D* plan) {
     const bool per = s->periodic_z != 0;
     const int nx = s->nx, nz = s->nz, npx = s->npml_x, npz = per ? 0 : s->npml_z;
     const int pitch = (nx + 31) & ~31;
-    // defaults from the variant / depth sweeps on the 4000 x 1500 workload
+    // defaults from variant / depth sweeps, us per step.  FP32 on 4000 x 1500:
+    // variant 1 at T = 8 25.5 (T = 6 26.9, T = 10 35.0, variant 2 34.2).  FP64
+    // on 800 x 300 / 1611 x 707: variant 2 at T = 8 5.08 / 11.5 (T = 6 5.46 /
+    // 11.9, T = 10 5.54 / 11.9, variant 1 at T = 8 6.55 / 13.2).
     const int fvariant = tuning.variant > 0 ? tuning.variant : (f64 ? 2 : 1);
     Variant2D fv, pv;
     if (!fast2d_info(fvariant, f64, false, &fv)) {
@@ -84,7 +87,7 @@ int plan2d(const orf_sim2d* s, const orf_tuning& tuning, Plan2D* plan) {
     fast2d_info(0, f64, true, &pv);
     // a tile's output keeps T cells (plus up to 3 of x alignment) from its edges
     const int tmax = std::min({kMaxSub, (pv.lz() - 1) / 2, (pv.lx() - 4) / 2, (fv.lz() - 1) / 2, (fv.lx() - 4) / 2});
-    int T = tuning.tsteps > 0 ? tuning.tsteps : (f64 ? 6 : 8);
+    int T = tuning.tsteps > 0 ? tuning.tsteps : 8;
     if (T > tmax) T = tmax;
     if (T < 1) T = 1;
 
