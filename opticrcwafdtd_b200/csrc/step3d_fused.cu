@@ -79,18 +79,38 @@ __device__ __forceinline__ int slab(bool half, int u, int n, int np) {
 }
 
 // CPML context of one instance, staged in shared memory by the CPML launches
-// so that a stretched difference costs one psi load, not a chain of
-// dependent descriptor loads.  kind 0: E update (integer positions, psiE),
-// kind 1: H update (half positions, psiH).
+// so that a stretched difference costs no chain of dependent descriptor
+// loads.  kind 0: E update (integer positions, psiE), kind 1: H update (half
+// positions, psiH).
+template <class R>
+struct alignas(2 * sizeof(R)) Prof3 {
+    R b, a;
+};
 template <class R>
 struct Cpml3 {
-    const R* prof[2][3];        // (b, a, 1/kappa) per coordinate, per axis
+    const R* prof[2][3];        // (b, a, 1/kappa) per coordinate, per axis (global memory)
+    // (b, a) of the tile's coordinates, one more on the low side
+    Prof3<R> px[2][TX + 1], py[2][TY + 1], pz[2][kSeg3 + 1];
+    int k0;                     // first plane of the tile's segment
     const R* pin[2][3][3];      // psi of (component, axis), buffer par (read)
     R* pout[2][3][3];           // the same, buffer par^1 (written)
     int n[3], np[3], nsl[2][3];
-    const R* zp[2];             // z profile of the segment's planes zk0 .. in shared memory
-    int zk0;
+    unsigned st[2][3];          // psi entries from one plane (x, y) or slab plane (z) to the next
 };
+
+// One column's place in the psi arrays of one update kind: the entry of plane
+// k is x + k st[0] and y + k st[1] (negative: the column is off the slab of
+// that axis), of z slab plane s it is z + s st[2]; rx, ry: the column in the
+// tile's E region (the low halo is 0), where its profile entries are.
+struct Col3 {
+    int x, y, z, rx, ry;
+};
+template <class R>
+__device__ __forceinline__ Col3 col3(const Cpml3<R>& X, int kind, int i, int j, int rx, int ry) {
+    const bool half = kind == 1;
+    const int sx = slab(half, i, X.n[0], X.np[0]), sy = slab(half, j, X.n[1], X.np[1]);
+    return {sx < 0 ? -1 : sx + X.nsl[kind][0] * j, sy < 0 ? -1 : i + X.n[0] * sy, i + X.n[0] * j, rx, ry};
+}
 
 // The six differences of one cell's H or E update, in the order
 // (c, q) = (0,1) (0,2) (1,2) (1,0) (2,0) (2,1): component c, derivative axis q.
@@ -99,25 +119,32 @@ struct Cpml3 {
 // axis by axis: the two psi loads of an axis are issued together, and a cell
 // on the slab of a single axis (all but the slab corners) has all its psi
 // loads in flight at once.  psi of buffer par is read-only during the launch.
-// zpre: z0, z1 are this cell's two z-axis psi values, loaded ahead by the
-// caller (the same values the loads here would return).
+// sz: slab plane of k on the z axis (-1: none); zpre: z0, z1 are this cell's
+// two z-axis psi values, loaded ahead by the caller (the same values the loads
+// here would return).  The offsets fit 32 bits: a psi array of 2^32 entries
+// would belong to fields larger than the device memory.
+// A CPML plane is a chain of about 400 instructions per warp (interior: 200) at
+// 13 cycles each, so instructions count: with the offsets hoisted per column
+// and (b, a) pairs in shared memory, against 64-bit offsets worked out for
+// every access and profiles read from global memory, the CPML launch of a 201
+// x 93 x 77 FP32 grid takes 62 us instead of 70, that of 600 x 600 x 300 457
+// instead of 495.  (Reading all psi of a plane at its top, in flight together,
+// costs more in registers than it hides: 68 and 531.  The FP32 ring leaves 0.4
+// KB of shared memory at three CTAs per SM; with two, 94 and 544.)
 template <class R>
-__device__ __forceinline__ void cpml6(const Cpml3<R>& X, int kind, bool store, int i, int j, int k, R (&d)[6],
-                                      bool zpre = false, R z0 = R(0), R z1 = R(0)) {
-    const bool half = kind == 1;
+__device__ __forceinline__ void cpml6(const Cpml3<R>& X, int kind, bool store, const Col3& col, int k, int sz,
+                                      R (&d)[6], bool zpre = false, R z0 = R(0), R z1 = R(0)) {
+    static_assert(kUnitKappa, "the stretched difference is d + psi");
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        const int coord = q == 0 ? i : (q == 1 ? j : k);
-        const int sl = slab(half, coord, X.n[q], X.np[q]);
-        if (sl < 0) continue;
         // the entries on axis q: (component c1, entry e1), (c2, e2)
         constexpr int E1[3] = {3, 0, 1}, E2[3] = {4, 5, 2};
         constexpr int C1[3] = {1, 0, 0}, C2[3] = {2, 2, 1};
-        const int v0 = q == 0 ? sl : i, v1 = q == 1 ? sl : j, v2 = q == 2 ? sl : k;
-        const int d0 = q == 0 ? X.nsl[kind][0] : X.n[0], d1 = q == 1 ? X.nsl[kind][1] : X.n[1];
-        const size_t o = (size_t)v0 + (size_t)d0 * ((size_t)v1 + (size_t)d1 * v2);
-        const bool zs = q == 2 && X.zp[kind] != nullptr;   // z profile staged in shared memory
-        const R* pr = zs ? X.zp[kind] + 3 * (coord - X.zk0) : X.prof[kind][q] + 3 * coord;
+        if ((q == 0 ? col.x : (q == 1 ? col.y : sz)) < 0) continue;
+        const unsigned o = q == 0   ? (unsigned)col.x + (unsigned)k * X.st[kind][0]
+                           : q == 1 ? (unsigned)col.y + (unsigned)k * X.st[kind][1]
+                                    : (unsigned)col.z + (unsigned)sz * X.st[kind][2];
+        const Prof3<R> pr = q == 0 ? X.px[kind][col.rx] : (q == 1 ? X.py[kind][col.ry] : X.pz[kind][k - X.k0 + 1]);
         R ps1, ps2;
         if (q == 2 && zpre) {
             ps1 = z0;
@@ -126,24 +153,14 @@ __device__ __forceinline__ void cpml6(const Cpml3<R>& X, int kind, bool store, i
             ps1 = __ldg(X.pin[kind][C1[q]][q] + o);
             ps2 = __ldg(X.pin[kind][C2[q]][q] + o);
         }
-        R b, a, ki = R(1);
-        if (zs) {
-            b = pr[0];
-            a = pr[1];
-            if (!kUnitKappa) ki = pr[2];
-        } else {
-            b = __ldg(pr);
-            a = __ldg(pr + 1);
-            if (!kUnitKappa) ki = __ldg(pr + 2);
-        }
-        const R p1 = b * ps1 + a * d[E1[q]];
-        const R p2 = b * ps2 + a * d[E2[q]];
+        const R p1 = pr.b * ps1 + pr.a * d[E1[q]];
+        const R p2 = pr.b * ps2 + pr.a * d[E2[q]];
         if (store) {
             X.pout[kind][C1[q]][q][o] = p1;
             X.pout[kind][C2[q]][q][o] = p2;
         }
-        d[E1[q]] = kUnitKappa ? d[E1[q]] + p1 : d[E1[q]] * ki + p1;
-        d[E2[q]] = kUnitKappa ? d[E2[q]] + p2 : d[E2[q]] * ki + p2;
+        d[E1[q]] = d[E1[q]] + p1;
+        d[E2[q]] = d[E2[q]] + p2;
     }
 }
 
@@ -228,14 +245,14 @@ __device__ __forceinline__ void tma_load3(void* sdst, const void* tmap, int x, i
 template <bool PML, class R>
 __device__ __forceinline__ void h_cell(const Inst3D<R>* __restrict__ I, const Cpml3<R>& X, bool store, int i, int j,
                                        int k, R ex, R ey, R ez, R ex_k, R ey_k, R ez_i, R ey_i, R ez_j, R ex_j, R& hx,
-                                       R& hy, R& hz, R gE, bool src, bool zpre = false, R z0 = R(0),
-                                       R z1 = R(0)) {
+                                       R& hy, R& hz, R gE, bool src, const Col3& col, int sz,
+                                       bool zpre = false, R z0 = R(0), R z1 = R(0)) {
     const R C = I->C;
     // Hx -= C ((Ez(j+1) - Ez) - (Ey(k+1) - Ey))
     // Hy -= C ((Ex(k+1) - Ex) - (Ez(i+1) - Ez))
     // Hz -= C ((Ey(i+1) - Ey) - (Ex(j+1) - Ex))
     R dd[6] = {ez_j - ez, ey_k - ey, ex_k - ex, ez_i - ez, ey_i - ey, ex_j - ex};
-    if (PML) cpml6(X, 1, store, i, j, k, dd, zpre, z0, z1);
+    if (PML) cpml6(X, 1, store, col, k, sz, dd, zpre, z0, z1);
     hx = hx - C * (dd[0] - dd[1]);
     hy = hy - C * (dd[2] - dd[3]);
     hz = hz - C * (dd[4] - dd[5]);
@@ -336,28 +353,29 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     __syncthreads();
-    // CPML tiles: the z profile (b, a, 1/kappa) of planes k0-1 .. k1 in shared
-    // memory, the entry every cell of a plane reads
-    __shared__ R szp[PML ? 2 : 1][PML ? 3 * (kSeg3 + 2) : 1];
     const int np2 = PML ? sx.np[2] : 0;
     // FP32 CPML tiles with a z slab on the TMA path take the z-axis psi of
     // their cells through the ring as well (slab planes of the psi arrays)
     const bool zring = ZR && use_tma && I->tma_psi != 0 && np2 > 0;
     const unsigned tx_bytes = kTx + (zring ? 4u * (unsigned)(SX * RY * sizeof(R)) : 0u);
     if constexpr (PML) {
-        const int cnt = k1 - k0 + 2;
-        if (np2 > 0) {
-            for (int q = t; q < 6 * cnt; q += NT) {
-                const int kind = q / (3 * cnt), r = q - kind * 3 * cnt, c = r / 3 + k0 - 1, f = r - 3 * (r / 3);
-                szp[kind][r] = (c >= 0 && c < nz) ? sx.prof[kind][2][3 * c + f] : R(f == 1 ? 0 : 1);
+        // the profiles of the tile's coordinates
+        const int u0[3] = {i0 - 1, j0 - 1, k0 - 1}, cnt[3] = {TX + 1, TY + 1, k1 - k0 + 1};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (sx.np[q] <= 0) continue;
+            for (int e = t; e < 2 * cnt[q]; e += NT) {
+                const int kind = e / cnt[q], r = e - kind * cnt[q], c = r + u0[q];
+                Prof3<R> v{R(1), R(0)};
+                if (c >= 0 && c < sx.n[q]) v = {sx.prof[kind][q][3 * c], sx.prof[kind][q][3 * c + 1]};
+                (q == 0 ? sx.px[kind] : (q == 1 ? sx.py[kind] : sx.pz[kind]))[r] = v;
             }
+            if (t < 2)
+                sx.st[t][q] = q == 0   ? (unsigned)sx.nsl[t][0] * (unsigned)sx.n[1]
+                              : q == 1 ? (unsigned)sx.n[0] * (unsigned)sx.nsl[t][1]
+                                       : (unsigned)sx.n[0] * (unsigned)sx.n[1];
         }
-        __syncthreads();   // every thread has read sx.np
-        if (t == 0) {
-            sx.zk0 = k0 - 1;
-            sx.zp[0] = np2 > 0 ? &szp[0][0] : nullptr;
-            sx.zp[1] = np2 > 0 ? &szp[1][0] : nullptr;
-        }
+        if (t == 0) sx.k0 = k0;
         __syncthreads();
     }
 
@@ -488,7 +506,8 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
             const R ez_j = jok ? __ldg(Ein[2] + oj) : R(0), ex_j = jok ? __ldg(Ein[0] + oj) : R(0);
             R hx = __ldg(Hin[0] + o), hy = __ldg(Hin[1] + o), hz = __ldg(Hin[2] + o);
             h_cell<PML>(I, sx, false, i, j, km, ex, ey, ez, ex_k, ey_k, ez_i, ey_i, ez_j, ex_j, hx, hy, hz, gE,
-                        sel3(I->sa, i, j, km) == I->ss - 1);
+                        sel3(I->sa, i, j, km) == I->ss - 1, PML ? col3(sx, 1, i, j, tx + 1, ty + 1) : Col3{},
+                        PML ? slab(true, km, nz, np2) : -1);
             hxm = hx;
             hym = hy;
         }
@@ -536,6 +555,19 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
     // (FP32: in FP64 the values held ahead would spill at three CTAs per SM)
     const bool zpre = PML && sizeof(R) == 4 && np2 > 0 && !zring;
     const bool zgiven = zpre || zring;   // the z-axis psi reach cpml6 from outside
+    // own cell H, own cell E, halo cell H (FP64 works them out at each use: held
+    // along the march they spill, and a 200 x 160 x 141 step takes 205 us instead
+    // of 199)
+    Col3 colO{}, colE{}, colH{};
+    if constexpr (PML && sizeof(R) == 4) {
+        colO = col3(sx, 1, i, j, tx + 1, ty + 1);
+        colE = col3(sx, 0, i, j, tx + 1, ty + 1);
+        colH = col3(sx, 1, hi, hj, hc, hr);
+    }
+    auto column = [&](const Col3& held, int kind, int ci, int cj, int rx, int ry) {
+        if constexpr (PML && sizeof(R) == 8) return col3(sx, kind, ci, cj, rx, ry);
+        else return held;
+    };
     R zHo0 = R(0), zHo1 = R(0), zHh0 = R(0), zHh1 = R(0), zEo0 = R(0), zEo1 = R(0);
     auto load_zH = [&](int p) {
         const int sl = slab(true, p, nz, np2);
@@ -572,6 +604,7 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
         const R* H0x = sHq(s0, 0);
         const R* H0y = sHq(s0, 1);
         const R* H0z = sHq(s0, 2);
+        const int szH = PML ? slab(true, k, nz, np2) : -1, szE = PML ? slab(false, k, nz, np2) : -1;
         // ---- H of plane k: the halo cell (its psi reads issued ahead of the
         // own cell's psi writes), then the own cell
         if (hasHalo) {
@@ -582,7 +615,8 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
                 hy = H0y[e];
                 hz = H0z[e];
                 h_cell<PML>(I, sx, false, hi, hj, k, E0x[e], E0y[e], E0z[e], E1x[e], E1y[e], E0z[e + 1], E0y[e + 1],
-                            E0z[e + SX], E0x[e + SX], hx, hy, hz, gE, SP && (haloSrcH || k == kSrcH), zgiven,
+                            E0z[e + SX], E0x[e + SX], hx, hy, hz, gE, SP && (haloSrcH || k == kSrcH),
+                            column(colH, 1, hi, hj, hc, hr), szH, zgiven,
                             zring ? sZq(s0, 0)[e] : zHh0, zring ? sZq(s0, 1)[e] : zHh1);
             }
             sHn[e] = hx;
@@ -601,7 +635,8 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
                 hyk = H0y[e];
                 hzk = H0z[e];
                 h_cell<PML>(I, sx, true, i, j, k, exo, eyo, ezo, E1x[e], E1y[e], E0z[e + 1], E0y[e + 1], E0z[e + SX],
-                            E0x[e + SX], hxk, hyk, hzk, gE, SP && (ownSrcH || k == kSrcH), zgiven,
+                            E0x[e + SX], hxk, hyk, hzk, gE, SP && (ownSrcH || k == kSrcH),
+                            column(colO, 1, i, j, tx + 1, ty + 1), szH, zgiven,
                             zring ? sZq(s0, 0)[e] : zHo0, zring ? sZq(s0, 1)[e] : zHo1);
                 const size_t o = (size_t)k * plane + (size_t)j * pitch + i;
                 Hout[0][o] = hxk;
@@ -625,7 +660,8 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
             // Ez += cz ((Hy - Hy(i-1)) - (Hx - Hx(j-1)))
             R dd[6] = {hzk - hz_j, hyk - hym, hxk - hxm, hzk - hz_i, hyk - hy_i, hxk - hx_j};
             if (PML)
-                cpml6(sx, 0, true, i, j, k, dd, zgiven, zring ? sZq(s0, 2)[e] : zEo0, zring ? sZq(s0, 3)[e] : zEo1);
+                cpml6(sx, 0, true, column(colE, 0, i, j, tx + 1, ty + 1), k, szE, dd, zgiven,
+                      zring ? sZq(s0, 2)[e] : zEo0, zring ? sZq(s0, 3)[e] : zEo1);
             R ex = exo + coef<R, IT>(slut, I->lutc, v0) * (dd[0] - dd[1]);
             R ey = eyo + coef<R, IT>(slut, I->lutc, v1) * (dd[2] - dd[3]);
             R ez = ezo + coef<R, IT>(slut, I->lutc, v2) * (dd[4] - dd[5]);
