@@ -74,10 +74,10 @@ int plan2d(const orf_sim2d* s, const orf_tuning& tuning, Plan2D* plan) {
     const bool per = s->periodic_z != 0;
     const int nx = s->nx, nz = s->nz, npx = s->npml_x, npz = per ? 0 : s->npml_z;
     const int pitch = (nx + 31) & ~31;
-    // defaults from variant / depth sweeps, us per step.  FP32 on 4000 x 1500:
-    // variant 1 at T = 8 25.5 (T = 6 26.9, T = 10 35.0, variant 2 34.2).  FP64
-    // on 800 x 300 / 1611 x 707: variant 2 at T = 8 5.08 / 11.5 (T = 6 5.46 /
-    // 11.9, T = 10 5.54 / 11.9, variant 1 at T = 8 6.55 / 13.2).
+    // defaults from variant / depth sweeps, us per step.  FP32, 32 runs of 800
+    // x 300 together: variant 1 at T = 8 50.4 (T = 6 53.1, T = 10 51.3, variant
+    // 2 59.3); on 4000 x 1500 25.0 (27.3, 34.0, 31.9).  FP64 on 800 x 300:
+    // variant 2 at T = 8 4.6 (T = 6 5.2, variant 1 at T = 8 6.0).
     const int fvariant = tuning.variant > 0 ? tuning.variant : (f64 ? 2 : 1);
     Variant2D fv, pv;
     if (!fast2d_info(fvariant, f64, false, &fv)) {

@@ -19,10 +19,11 @@ struct VDesc {
 // so short strips among many warps shorten a tile as long as the strip's state
 // fits the registers (64 for 1024 threads): 32 warps in the interior and 20 in
 // the frame, against 16 and 10 with strips twice as long, in us per step at
-// T = 8: FP64 601 x 4 (frame only) 6.4 -> 5.1, 800 x 300 TE 6.9 -> 5.1, 1611 x
-// 707 TM 12.3 -> 11.5; FP32 4000 x 1500 TM 26.5 -> 25.5, 32 runs of 800 x 300
-// together 73.8 -> 61.2.  (FP32 frame tiles on one CTA per SM, unspilled: the
-// batch 64.8; a single 800 x 300 run is the same.)
+// T = 8: FP64 601 x 4 6.4 -> 5.1, 800 x 300 TE 6.9 -> 5.1, 1611 x 707 TM 12.3
+// -> 11.5; FP32 4000 x 1500 TM 26.5 -> 25.5, 32 runs of 800 x 300 together 73.8
+// -> 61.2 (FP32 frame tiles on one CTA per SM, unspilled: 64.8).  With the
+// samples' and the source's data in shared memory and the monitor addresses
+// out of the interior's registers these are 3.7, 4.6, 11.3, 23.3 and 50.4.
 constexpr VDesc kF32[] = {{1, 8, 4, 8}, {2, 4, 4, 8}};
 constexpr VDesc kF64[] = {{1, 4, 4, 8}, {2, 4, 2, 16}};
 // CPML / boundary tiles: 64 x 40 covers a (npml + T)-cell frame strip in

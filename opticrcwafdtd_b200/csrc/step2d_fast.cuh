@@ -114,6 +114,14 @@ constexpr size_t dyn_smem() {
     return b;
 }
 
+// where a tile's monitor samples go (Inst2D)
+template <class R>
+struct MonCtx {
+    R* samples;
+    int sstride, nmon, nmonz;
+    int monz[kMaxMon];
+};
+
 // 16 bytes of an exchange row (16-byte aligned) into registers
 template <class R>
 __device__ __forceinline__ void load16(R (&dst)[16 / sizeof(R)], const R* src) {
@@ -172,6 +180,14 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
     __shared__ R slut[256];
     __shared__ const R* s_lutsrc;
     __shared__ double sg[2][kMaxSub];
+    // tiles with the TF/SF plane: the source profile (B, P) of the loaded rows,
+    // zero outside the grid; tiles with monitors: where their samples go.  Read
+    // in every fused step: from global memory, through the instance record,
+    // they made such a tile up to half as slow again as a plain one, and a
+    // launch of a single wave waits for it (us per step: 601 x 4 FP64 5.1 ->
+    // 3.7, 800 x 300 FP64 5.1 -> 4.6, 32 runs of 800 x 300 FP32 61 -> 58.5)
+    __shared__ R s_src[2][LZ];
+    __shared__ MonCtx<R> s_mon;
     __shared__ double sred[NW];
     // descriptor ring (tiles t, t+G, t+2G) and snapshots of their job state,
     // both filled by cp.async so no thread waits on a dependent global load
@@ -307,10 +323,29 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
             __syncthreads();
             if (threadIdx.x == 0) s_lutsrc = I->lutc;
         }
-        for (int q = threadIdx.x; q < nsub; q += NT) {
-            const long long n = n0 + q;
-            sg[0][q] = n < I->nsrc ? I->gE[n] : 0.0;
-            sg[1][q] = n < I->nsrc ? I->gH[n] : 0.0;
+        if (d.flags & 1) {
+            for (int q = threadIdx.x; q < nsub; q += NT) {
+                const long long n = n0 + q;
+                sg[0][q] = n < I->nsrc ? I->gE[n] : 0.0;
+                sg[1][q] = n < I->nsrc ? I->gH[n] : 0.0;
+            }
+            // (the loaded rows may run past the grid's last row: the source
+            // profile is read for grid rows only)
+            for (int q = threadIdx.x; q < LZ; q += NT) {
+                const int kk = d.periodic ? pmod(d.lk0 + q, d.nz) : d.lk0 + q;
+                const bool v = kk >= 0 && kk < d.nz && ORF_IN(kk, d.nz);
+                s_src[0][q] = v ? I->srcB[kk] : R(0);
+                s_src[1][q] = v ? I->srcP[kk] : R(0);
+            }
+        }
+        if (d.flags & 6) {
+            if (threadIdx.x < kMaxMon) s_mon.monz[threadIdx.x] = I->monz[threadIdx.x];
+            if (threadIdx.x == kMaxMon) {
+                s_mon.samples = I->samples;
+                s_mon.sstride = I->sstride;
+                s_mon.nmon = I->nmon;
+                s_mon.nmonz = I->nmonz;
+            }
         }
         const int i = d.li0 + cx;
         const int kb = d.lk0 + ck0;
@@ -419,19 +454,28 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
 #pragma unroll
             for (int j = 0; j < KS; ++j)
                 if (colown && kb + j >= d.ok0 && kb + j < d.ok0 + d.oh) own |= 1u << j;
-            const bool hs = (d.flags & 1) != 0;   // tile holds the TF/SF plane
-            const int six = hs ? I->src_ix : -8;
-            int xm = -1;
-            unsigned zmask = 0;
+            // with the owned rows in one register through the steps: the owned
+            // rows a z monitor samples (bits 8 ..), the column's x monitor plus
+            // one (bits 16 ..) and whether the column is the one left of the
+            // TF/SF plane (bit 30) or the plane (bit 31)
+            static_assert(KS <= 8 && kMaxMon < 31, "packed masks");
+            if (d.flags & 1) {
+                const int six = I->src_ix;
+                if (i == six - 1) own |= 1u << 30;
+                if (i == six) own |= 1u << 31;
+            }
             if (d.flags & 2)
                 for (int m = 0; m < I->nmon; ++m)
-                    if (I->mon[m] == i) { xm = m; break; }
+                    if (I->mon[m] == i) {
+                        own |= (unsigned)(m + 1) << 16;
+                        break;
+                    }
             if (d.flags & 4) {
 #pragma unroll
                 for (int j = 0; j < KS; ++j) {
                     const int kk = d.periodic ? pmod(kb + j, d.nz) : kb + j;
                     for (int m = 0; m < I->nmonz; ++m)
-                        if (I->monz[m] == kk) zmask |= ((own >> j) & 1u) << j;
+                        if (I->monz[m] == kk) own |= ((own >> j) & 1u) << (8 + j);
                 }
             }
             R pxb = R(1), pxa = R(0), pxk = R(1), phb = R(1), pha = R(0), phk = R(1);
@@ -486,16 +530,11 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
                             B[j] = fma(-cb, dx, B[j]);
                         }
                     }
-                    // (an interior tile has no row masks, and its loaded rows
-                    // may run past the grid's last row: the source profile is
-                    // read for grid rows only)
-                    if (hs && i == six - 1) {   // TF/SF: the B column left of the plane is scattered field
+                    if ((own >> 30) & 1u) {   // TF/SF: the B column left of the plane is scattered field
                         const R ge = (R)sg[0][s];
     #pragma unroll
                         for (int j = 0; j < KS; ++j) {
-                            const int kk = d.periodic ? pmod(kb + j, nz) : kb + j;
-                            if (((mB >> j) & 1u) && kk >= 0 && kk < nz && ORF_IN(kk, nz))
-                                B[j] = fma(__ldg(I->srcB + kk), ge, B[j]);
+                            if ((mB >> j) & 1u) B[j] = fma(s_src[0][ck0 + j], ge, B[j]);
                         }
                     }
                     // ----- E half step: P (branch-free stencil loop)
@@ -534,43 +573,52 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
                         }
                     }
                     // rare paths, each behind a tile-uniform flag
-                    if (hs && i == six) {   // TF/SF: the plane is total field
+                    if (own >> 31) {   // TF/SF: the plane is total field
                         const R gh = (R)sg[1][s];
     #pragma unroll
                         for (int j = 0; j < KS; ++j) {
-                            const int kk = d.periodic ? pmod(kb + j, nz) : kb + j;
-                            if (((mP >> j) & 1u) && kk >= 0 && kk < nz && ORF_IN(kk, nz))
-                                P[j] = fma(__ldg(I->srcP + kk), gh, P[j]);
+                            if ((mP >> j) & 1u) P[j] = fma(s_src[1][ck0 + j], gh, P[j]);
                         }
                     }
                     if (d.flags & 6) {      // DFT monitor samples of this step
+                        // FP32 interior tiles: worked out anew in each step.  Hoisted
+                        // out of the loop, the addresses of this path hold registers
+                        // that the 64 of a thread do not have: 35 spilled instead of
+                        // 10, and an interior launch of 4000 x 1500 TM takes 159 us
+                        // instead of 141 (FP64: 71 us against 74 on 1611 x 707)
+                        int kq = kb, iq = i;
+                        unsigned ownq = own;
+                        if (!PML && sizeof(R) == 4) asm volatile("" : "+r"(kq), "+r"(iq), "+r"(ownq));
+                        const int xmq = (int)((ownq >> 16) & 31u) - 1;
                         const int sslot = launch_off + s;
-                        R* smp0 = I->samples + (size_t)sslot * I->sstride;
+                        const int sstride = s_mon.sstride;
+                        R* smp0 = s_mon.samples + (size_t)sslot * sstride;
     #pragma unroll
                         for (int j = 0; j < KS; ++j) {
                             if (j % VEC == 0) load16<R>(be, &xBc[wL][j]);
                             R bl = __shfl_up_sync(FULL, B[j], 1);
                             const R bej = (PML && !hasL) ? R(0) : be[j % VEC];
                             bl = (lane == 0) ? bej : bl;
-                            if (xm >= 0 && ((own >> j) & 1u)) {
-                                R* smp = smp0 + (size_t)xm * 2 * nz;
-                                if (ORF_IN((size_t)sslot * I->sstride + (size_t)xm * 2 * nz + nz + kb + j,
-                                           (size_t)kChunk * I->sstride)) {
-                                    smp[kb + j] = P[j];
-                                    smp[nz + kb + j] = R(0.5) * (bl + B[j]);
+                            if (xmq >= 0 && ((ownq >> j) & 1u)) {
+                                R* smp = smp0 + (size_t)xmq * 2 * nz;
+                                if (ORF_IN((size_t)sslot * sstride + (size_t)xmq * 2 * nz + nz + kq + j,
+                                           (size_t)kChunk * sstride)) {
+                                    smp[kq + j] = P[j];
+                                    smp[nz + kq + j] = R(0.5) * (bl + B[j]);
                                 }
                             }
-                            if ((zmask >> j) & 1u) {
+                            if ((ownq >> (8 + j)) & 1u) {
                                 const R am = (j > 0) ? A[j - 1] : Aup;
-                                for (int m = 0; m < I->nmonz; ++m) {
-                                    if (I->monz[m] != kb + j) continue;
-                                    R* smp = smp0 + (size_t)I->nmon * 2 * nz + (size_t)m * 2 * d.nx;
-                                    if (!ORF_IN((size_t)sslot * I->sstride + (size_t)I->nmon * 2 * nz +
-                                                    (size_t)m * 2 * d.nx + d.nx + i,
-                                                (size_t)kChunk * I->sstride))
+                                const int nmon = s_mon.nmon, nmonz = s_mon.nmonz;
+                                for (int m = 0; m < nmonz; ++m) {
+                                    if (s_mon.monz[m] != kq + j) continue;
+                                    R* smp = smp0 + (size_t)nmon * 2 * nz + (size_t)m * 2 * d.nx;
+                                    if (!ORF_IN((size_t)sslot * sstride + (size_t)nmon * 2 * nz +
+                                                    (size_t)m * 2 * d.nx + d.nx + iq,
+                                                (size_t)kChunk * sstride))
                                         continue;
-                                    smp[i] = P[j];
-                                    smp[d.nx + i] = R(0.5) * (am + A[j]);
+                                    smp[iq] = P[j];
+                                    smp[d.nx + iq] = R(0.5) * (am + A[j]);
                                 }
                             }
                         }
