@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_factor(FdfdDev P, const FdSeg* _
     for (int u = 0; u < RS; ++u) a[u] = make_double2(0.0, 0.0);
     int par = 0;
 
+    cl.sync();   // every CTA of the cluster runs: its shared memory may be written
     for (int it = 0; it < seg.n; ++it) {
         const int b = seg.dir > 0 ? seg.a + it : seg.a + seg.n - 1 - it;
         if (col) {
@@ -530,6 +531,7 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_sweep(FdfdDev P, const FdSeg* __
     mv.warp = t >> 5;
     __shared__ double2 s_full[2][kFdMaxM];   // the vector multiplied, by step parity
     __shared__ double2 s_y[32];              // the own entries of the last product
+    cl.sync();   // every CTA of the cluster runs: its shared memory may be written
     const int d = seg.dir, first = d > 0 ? seg.a : seg.a + seg.n - 1;
     // couplings of line b to the one before (prev) and after it, in the order of elimination
     auto e_prev = [&](int b) { return P.eb + (size_t)(d > 0 ? b : b + 1) * m; };
@@ -629,6 +631,7 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_red(FdfdDev P, FdRed D, const do
     mv.warp = t >> 5;
     __shared__ double2 s_full[2][kFdMaxM];
     __shared__ double2 s_y[32];
+    cl.sync();   // every CTA of the cluster runs: its shared memory may be written
     const int npush = mv.nr * C;
     int par = 0;
     constexpr int NPU = ((NQ > 8 ? 24 * 16 : 32 * 8) + NT - 1) / NT;
