@@ -57,7 +57,7 @@ struct FdfdDev {
     const double2* wc;         // [nb][m]: coupling of p - 1 and p inside the line (entry 0 unused)
     const double2* eb;         // [nb][m]: coupling of line b - 1 and b at p (line 0 unused)
     double2* inv;              // [nb][m][m]: D_b^{-1}, row-major
-    int* fault;                // a zero pivot (singular block)
+    int* fault;                // a zero or NaN pivot (singular block, permittivity that is not a number)
     double2* xrow;             // [clusters][kPanel][m]: pivot rows of a panel
 };
 
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_factor(FdfdDev P, const FdSeg* _
                         pr[l] = cfma(g, prw[l], base);
                     }
                     pr[aa] = g;
-                    if (me && dd == 0.0) atomicExch(P.fault, 1);   // a zero pivot
+                    if (me && !(dd > 0.0)) atomicExch(P.fault, 1);   // a zero or NaN pivot
                 }
                 if (t >= r0 && t < r0 + nr) {
                     s_kown[t - r0] = (signed char)myk;
@@ -1237,7 +1237,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         if (singular || !(eta <= kEtaTrial)) ORF_TRY(F->factor(1, &singular));
     }
     if (singular) {
-        set_error("fdfd2D: the operator is singular (a zero pivot in the block elimination)");
+        set_error("fdfd2D: the operator is singular (a zero or NaN pivot in the block elimination)");
         return ORF_EINVAL;
     }
     *out = F.release();

@@ -105,3 +105,14 @@ def test_fdfd_segment_in_resonance():
     assert rel(o.E, r.E) <= TOL
     assert rel(o.adjoint(J), r.adjoint(J)) <= TOL
     o.close()
+
+
+@pytest.mark.parametrize("nx,nz", [(12, 9), (170, 60), (90, 240)])
+def test_fdfd_refuses_a_permittivity_that_is_not_a_number(nx, nz):
+    """One NaN cell makes every pivot row NaN sooner or later: refused as a
+    singular operator, as one segment (12 x 9) and as many."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(nx, nz, 5, True, npml=(3, 3))
+    eps[nx // 2, nz // 3] = np.nan
+    with pytest.raises(orf.OrfError) as ei:
+        orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    assert ei.value.identifier == "orf:invalidInput"
