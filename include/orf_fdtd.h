@@ -485,6 +485,9 @@ ORF_API int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* problem, orf_f
 ORF_API int32_t orf_fdfd2d_solve(orf_fdfd* f, const double* rhs, double* x, int32_t transpose);
 /* block size (shorter axis), number of blocks, CTAs of the solver's cluster */
 ORF_API int32_t orf_fdfd2d_info(const orf_fdfd* f, int32_t* block, int32_t* nblocks, int32_t* cluster);
+/* segments the lines were to be cut into, and those of the factors (1 where
+ * a segment turned out nearly singular by itself, or memory was short) */
+ORF_API int32_t orf_fdfd2d_segments(const orf_fdfd* f, int32_t* planned, int32_t* segments);
 ORF_API void    orf_fdfd2d_release(orf_fdfd* f);
 
 #ifdef __cplusplus

@@ -897,7 +897,7 @@ struct orf_fdfd {
     orf_ctx* ctx = nullptr;
     int nx = 0, nz = 0, m = 0, nb = 0, C = 8;
     bool along_x = true;   // blocks are lines of constant x (m = nz)
-    int S = 1;             // segments
+    int S = 1, planned = 1;   // segments of the factors, and as chosen for the grid
     double mnorm = 0.0;    // bound of the row sums of |M|
     Arena ar;
     double2 *diag = nullptr, *wc = nullptr, *eb = nullptr, *sx = nullptr, *sz = nullptr;
@@ -1176,6 +1176,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         ORF_CUDA(launch_factor(P, F->C, nullptr, 1, st, &most));
     }
     int S = fd_segments(nb, most);
+    F->planned = S;
     Arena& ar = F->ar;
     auto carve = [&]() {
         const int J = S - 1;
@@ -1294,5 +1295,15 @@ extern "C" int32_t orf_fdfd2d_info(const orf_fdfd* F, int32_t* block, int32_t* n
     if (block) *block = F->m;
     if (nblocks) *nblocks = F->nb;
     if (cluster) *cluster = F->C;
+    return ORF_OK;
+}
+
+extern "C" int32_t orf_fdfd2d_segments(const orf_fdfd* F, int32_t* planned, int32_t* segments) {
+    if (!F) {
+        set_error("fdfd handle is null");
+        return ORF_EINVAL;
+    }
+    if (planned) *planned = F->planned;
+    if (segments) *segments = F->S;
     return ORF_OK;
 }

@@ -72,7 +72,10 @@ class FDFD2D:
     def info(self) -> dict:
         m, nb, cl = C.c_int32(), C.c_int32(), C.c_int32()
         _lib.check(self.lib.orf_fdfd2d_info(self.handle, C.byref(m), C.byref(nb), C.byref(cl)), "fdfd2D info")
-        return {"block": m.value, "blocks": nb.value, "cluster": cl.value}
+        planned, segs = C.c_int32(), C.c_int32()
+        _lib.check(self.lib.orf_fdfd2d_segments(self.handle, C.byref(planned), C.byref(segs)), "fdfd2D info")
+        return {"block": m.value, "blocks": nb.value, "cluster": cl.value, "planned_segments": planned.value,
+                "segments": segs.value}
 
     def _run(self, v, transpose: int) -> np.ndarray:
         if self.handle is None:

@@ -116,3 +116,45 @@ def test_fdfd_refuses_a_permittivity_that_is_not_a_number(nx, nz):
     with pytest.raises(orf.OrfError) as ei:
         orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
     assert ei.value.identifier == "orf:invalidInput"
+
+
+@pytest.mark.parametrize("nx,nz,cut", [(3, 5, False), (8, 6, False), (64, 90, True), (131, 129, True), (258, 257, True)])
+def test_fdfd_reports_its_segments(nx, nz, cut):
+    """The factors of an ordinary grid are those planned; grids of a hundred
+    lines are cut, the smallest are not."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(nx, nz, 2, True, npml=(min(8, (nx - 1) // 2),
+                                                                                min(6, (nz - 1) // 2)))
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    info = o.info()
+    o.close()
+    assert info["segments"] == info["planned_segments"]
+    assert (info["segments"] > 1) == cut
+
+
+@pytest.mark.parametrize("nb,planned", [(9, 2), (14, 3), (35, 6), (41, 7), (60, 9)])
+def test_fdfd_odd_and_even_separator_counts(nb, planned):
+    """Two to nine segments (one to eight separators, met in the middle from
+    both ends): odd and even counts, against the oracle."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(nb, 7, nb, True, npml=(2, 2))
+    J[nb // 3, 1:6] = 1.0 + 0.3j
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    r = oracle_fdfd2D(x, z, eps, lam, J, Npml=npml)
+    info = o.info()
+    assert info["planned_segments"] == planned and info["segments"] == planned
+    assert rel(o.E, r.E) <= TOL
+    assert rel(o.adjoint(g), r.adjoint(g)) <= TOL
+    o.close()
+
+
+def test_fdfd_segment_in_resonance_falls_back_to_one():
+    """The cavity of test_fdfd_segment_in_resonance: planned as seven
+    segments, five of them singular by themselves, factored as one."""
+    nx, nz, d, lam = 41, 6, 0.03, 1.3
+    ev = 4 / d ** 2 * (np.sin(np.pi / (2 * 6)) ** 2 + np.sin(np.pi / (2 * 7)) ** 2)
+    eps = np.full((nx, nz), ev / (2 * np.pi / lam) ** 2)
+    eps[:5] *= 1.3
+    eps[36:] *= 1.5
+    o = orf.fdfd2D(np.arange(nx) * d, np.arange(nz) * d, eps, lam, np.ones((nx, nz)), Npml=(0, 0))
+    info = o.info()
+    o.close()
+    assert info["planned_segments"] == 7 and info["segments"] == 1
