@@ -798,15 +798,19 @@ int fd_shape(int m, int* C) {
     return ORF_ETOOLARGE;
 }
 
+// limit: the most dynamic shared memory any launch of this kernel asks for (0:
+// none).  The attribute belongs to the kernel, not to a launch, so every launch
+// sets the same value: one that followed the block size would lower what
+// another host thread is about to launch with.
 template <class K, class... Args>
-cudaError_t launch_cluster(K kern, int clusters, int C, int threads, size_t smem, cudaStream_t s, int* most,
-                           Args... args) {
+cudaError_t launch_cluster(K kern, int clusters, int C, int threads, size_t smem, size_t limit, cudaStream_t s,
+                           int* most, Args... args) {
     if (C > 8) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
-    if (smem > 32 * 1024) {   // (the kernels' static arrays count too)
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (limit > 0) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -829,23 +833,24 @@ cudaError_t launch_cluster(K kern, int clusters, int C, int threads, size_t smem
 cudaError_t launch_factor(const FdfdDev& P, int C, const FdSeg* segs, int n, cudaStream_t s, int* most) {
     const int mp = (P.m + 31) / 32 * 32, R = (P.m + C - 1) / C;
     const size_t smem = fd_factor_smem(P.m, R);
-    if (C <= 4) return launch_cluster(k_fdfd_factor<8, 4, 512>, n, C, 4 * mp, smem, s, most, P, segs);
-    if (C == 8) return launch_cluster(k_fdfd_factor<16, 2, 512>, n, C, 2 * mp, smem, s, most, P, segs);
-    return launch_cluster(k_fdfd_factor<24, 1, 384>, n, C, mp, smem, s, most, P, segs);
+    // (the largest block of each kernel: fd_shape)
+    if (C <= 4) return launch_cluster(k_fdfd_factor<8, 4, 512>, n, C, 4 * mp, smem, fd_factor_smem(128, 32), s, most, P, segs);
+    if (C == 8) return launch_cluster(k_fdfd_factor<16, 2, 512>, n, C, 2 * mp, smem, fd_factor_smem(256, 32), s, most, P, segs);
+    return launch_cluster(k_fdfd_factor<24, 1, 384>, n, C, mp, smem, fd_factor_smem(kFdMaxM, 24), s, most, P, segs);
 }
 cudaError_t launch_sweep(const FdfdDev& P, int C, const FdSeg* segs, int n, const double2* f, double2* X, int seps,
                          cudaStream_t s) {
-    if (C == 2) return launch_cluster(k_fdfd_sweep<2, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
-    if (C == 4) return launch_cluster(k_fdfd_sweep<4, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
-    if (C == 8) return launch_cluster(k_fdfd_sweep<8, 2, 512>, n, C, 512, 0, s, nullptr, P, segs, f, X, seps);
-    return launch_cluster(k_fdfd_sweep<12, 2, 384>, n, C, 384, 0, s, nullptr, P, segs, f, X, seps);
+    if (C == 2) return launch_cluster(k_fdfd_sweep<2, 2, 512>, n, C, 512, 0, 0, s, nullptr, P, segs, f, X, seps);
+    if (C == 4) return launch_cluster(k_fdfd_sweep<4, 2, 512>, n, C, 512, 0, 0, s, nullptr, P, segs, f, X, seps);
+    if (C == 8) return launch_cluster(k_fdfd_sweep<8, 2, 512>, n, C, 512, 0, 0, s, nullptr, P, segs, f, X, seps);
+    return launch_cluster(k_fdfd_sweep<12, 2, 384>, n, C, 384, 0, 0, s, nullptr, P, segs, f, X, seps);
 }
 cudaError_t launch_red(const FdfdDev& P, int C, const FdRed& D, const double2* f, double2* X, int phase,
                        cudaStream_t s) {
-    if (C == 2) return launch_cluster(k_fdfd_red<2, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
-    if (C == 4) return launch_cluster(k_fdfd_red<4, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
-    if (C == 8) return launch_cluster(k_fdfd_red<8, 2, 512>, 2, C, 512, 0, s, nullptr, P, D, f, X, phase);
-    return launch_cluster(k_fdfd_red<12, 2, 384>, 2, C, 384, 0, s, nullptr, P, D, f, X, phase);
+    if (C == 2) return launch_cluster(k_fdfd_red<2, 2, 512>, 2, C, 512, 0, 0, s, nullptr, P, D, f, X, phase);
+    if (C == 4) return launch_cluster(k_fdfd_red<4, 2, 512>, 2, C, 512, 0, 0, s, nullptr, P, D, f, X, phase);
+    if (C == 8) return launch_cluster(k_fdfd_red<8, 2, 512>, 2, C, 512, 0, 0, s, nullptr, P, D, f, X, phase);
+    return launch_cluster(k_fdfd_red<12, 2, 384>, 2, C, 384, 0, 0, s, nullptr, P, D, f, X, phase);
 }
 
 // Segments for nb lines when `most` clusters run at once: the chain is

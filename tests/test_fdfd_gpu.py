@@ -1,6 +1,8 @@
 """orf.fdfd2D on the device (opticrcwafdtd_b200/fdfd.py, csrc/fdfd.cu) against
 the FDFD oracle, on the reference's own physics checks
 (tests/TestInverseDesign.m:12-33), and its adjoint gradient."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -158,3 +160,36 @@ def test_fdfd_segment_in_resonance_falls_back_to_one():
     info = o.info()
     o.close()
     assert info["planned_segments"] == 7 and info["segments"] == 1
+
+
+def test_fdfd_factorisations_on_several_threads():
+    """Blocks of 150 and of 250 points are factored by one kernel with
+    different shared memory sizes: side by side on two threads, each with its
+    own context, neither changes what the other may launch."""
+    probs = [fdfd_cases.random_problem(nx, nz, nx, True) for nx, nz in ((160, 150), (260, 250))]
+    first, got, errs = [], [[], []], []
+
+    def work(q, n):
+        x, z, eps, lam, J, g, npml = probs[q]
+        ctx = orf.Context(0)
+        try:
+            for _ in range(n):
+                o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml, ctx=ctx)
+                got[q].append((o.info()["segments"], o.E))
+                o.close()
+        except Exception as e:   # noqa: BLE001 (a thread's failure is the test's)
+            errs.append(e)
+        ctx.close()
+
+    for q in (0, 1):   # alone
+        work(q, 1)
+        first.append(got[q].pop())
+    th = [threading.Thread(target=work, args=(0, 150)), threading.Thread(target=work, args=(1, 60))]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not errs, errs
+    for q in (0, 1):
+        assert first[q][0] > 1
+        assert all(s == first[q][0] and np.array_equal(E, first[q][1]) for s, E in got[q])
