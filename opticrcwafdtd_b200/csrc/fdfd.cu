@@ -1210,7 +1210,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         return ar.alloc();
     };
     int rc = carve();
-    if (rc != ORF_OK && S > 1) {   // one segment needs no memory for separators
+    if (rc == ORF_ENOMEM_DEVICE && S > 1) {   // one segment needs no memory for separators
         S = 1;
         rc = carve();
     }
@@ -1226,7 +1226,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
     add_h2d(ctx, (int64_t)((3 * N + nx + nz) * sizeof(double2)));
     bool singular = false;
     rc = F->factor(S, &singular);
-    if (rc != ORF_OK && S > 1) {   // (no memory for the separators' blocks)
+    if (rc == ORF_ENOMEM_DEVICE && S > 1) {   // (the separators' blocks; every other error is the caller's to see)
         S = 1;
         rc = F->factor(S, &singular);
     }

@@ -40,3 +40,18 @@ def test_oracle_operator_is_the_documented_stencil():
     for q in (r - 1, r + 1, r - 30, r + 30):
         assert np.isclose(row[q], 1 / d ** 2)
     assert np.count_nonzero(row) == 5
+
+
+def test_only_a_lack_of_memory_is_retried_as_one_segment():
+    """orf_fdfd2d_factor goes on with one segment (many times slower) after an
+    error only where device memory was short; any other error is returned.
+    Read from the source: the failing calls cannot be made to fail here."""
+    import os
+    import re
+    import opticrcwafdtd_b200
+    src = open(os.path.join(os.path.dirname(opticrcwafdtd_b200.__file__), "csrc", "fdfd.cu")).read()
+    body = src[src.index("int32_t orf_fdfd2d_factor("):]
+    body = body[:body.index("\n}\n")]
+    retries = re.findall(r"if \(([^{]*)\) \{[^\n]*\n\s*S = 1;", body)
+    assert len(retries) == len(re.findall(r"\bS = 1;", body)) == 2
+    assert all(r == "rc == ORF_ENOMEM_DEVICE && S > 1" for r in retries), retries
