@@ -713,18 +713,47 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_red(FdfdDev P, FdRed D, const do
     cl.sync();   // no CTA leaves while another may still write its shared memory
 }
 
+// Power of two that brings the largest entry of a right-hand side to [1, 2):
+// its exponent (0 where there is none to take, an entry not finite or all zero).
+// big: the bits of the largest |re| or |im|.  A solve with it is the same to the
+// bit, and the squares in its residual neither vanish nor overflow.
+__device__ __forceinline__ int fd_exponent(const unsigned long long* big) {
+    const double v = big ? __longlong_as_double((long long)*big) : 0.0;
+    return v > 0.0 && v < CUDART_INF ? ilogb(v) : 0;
+}
+__device__ __forceinline__ double2 fd_scaled(double2 a, int e) {
+    return e == 0 ? a : make_double2(scalbn(a.x, e), scalbn(a.y, e));
+}
+__global__ void k_fd_biggest(const double2* __restrict__ v, size_t n, unsigned long long* big) {
+    double a = 0.0;
+    bool nan = false;
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+        const double2 x = v[o];
+        nan = nan || x.x != x.x || x.y != x.y;
+        a = fmax(a, fmax(fabs(x.x), fabs(x.y)));
+    }
+    if (nan) a = CUDART_INF;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(kFull, a, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(big, (unsigned long long)__double_as_longlong(a));
+}
+
 // The caller's vector (i + nx k) and the block layout (b m + p), with the
 // scaling by s = s_x(i) s_z(k): f = -s J (mode 0) or g (mode 1); E = x or s x.
+// big: the largest entry of the caller's vector, to whose scale f is brought
+// (null: f is not scaled).
 struct FdMap {
     int nx, nz, along_x;
     const double2 *sx, *sz;
     __device__ size_t at(int i, int k) const { return along_x ? (size_t)i * nz + k : (size_t)k * nx + i; }
 };
-__global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __restrict__ f, int mode) {
+__global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __restrict__ f, int mode,
+                        const unsigned long long* big) {
+    const int ex = fd_exponent(big);
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
          g += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
-        double2 x = v[g];
+        double2 x = fd_scaled(v[g], -ex);
         if (mode == 0) {
             x = cmul(cmul(mp.sx[i], mp.sz[k]), x);
             x = make_double2(-x.x, -x.y);
@@ -732,16 +761,18 @@ __global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __rest
         f[mp.at(i, k)] = x;
     }
 }
-__global__ void k_fd_out(FdMap mp, const double2* __restrict__ x, double2* __restrict__ v, int mode) {
+__global__ void k_fd_out(FdMap mp, const double2* __restrict__ x, double2* __restrict__ v, int mode,
+                         const unsigned long long* big) {
+    const int ex = fd_exponent(big);
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
          g += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
         const double2 y = x[mp.at(i, k)];
-        v[g] = mode == 0 ? y : cmul(cmul(mp.sx[i], mp.sz[k]), y);
+        v[g] = fd_scaled(mode == 0 ? y : cmul(cmul(mp.sx[i], mp.sz[k]), y), ex);
     }
 }
 // r = f - M x and the largest |r|^2, |x|^2 and |f|^2 (bits of non-negative
-// doubles order as integers); add: x += dx first
+// doubles order as integers)
 __global__ void k_fd_residual(FdfdDev P, const double2* __restrict__ f, const double2* __restrict__ x,
                               double2* __restrict__ r, unsigned long long* mx) {
     const size_t N = (size_t)P.nb * P.m;
@@ -909,7 +940,7 @@ struct orf_fdfd {
     double2 *inv = nullptr, *vin = nullptr, *vout = nullptr, *xrow = nullptr;
     double2 *f = nullptr, *x = nullptr, *r = nullptr, *dx = nullptr, *Y = nullptr, *YT = nullptr, *V = nullptr,
             *Z = nullptr;
-    unsigned long long* mx = nullptr;
+    unsigned long long* mx = nullptr;   // largest |r|^2, |x|^2, |f|^2; largest entry of the caller's right-hand side
     FdSeg* segs = nullptr;
     int *line = nullptr, *fault = nullptr;
     ~orf_fdfd() {
@@ -1202,7 +1233,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         ar.add(&F->YT, (size_t)J * m * m);
         ar.add(&F->V, (size_t)J * m);
         ar.add(&F->Z, (size_t)2 * m);
-        ar.add(&F->mx, 3);
+        ar.add(&F->mx, 4);
         ar.add(&F->segs, S);
         ar.add(&F->line, J);
         ar.add(&F->fault, 1);
@@ -1271,15 +1302,22 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
     } rel{stage, st};
     ORF_TRY(copy_h2d_staged(F->vin, rhs, bytes, stage, st));
     add_h2d(F->ctx, (int64_t)bytes);
-    k_fd_in<<<296, 256, 0, st>>>(F->map(), F->vin, F->f, mode);
+    const bool checked = F->S > 1;   // (as one segment: no residual is taken, nothing to scale for)
+    unsigned long long* big = checked ? F->mx + 3 : nullptr;
+    if (checked) {
+        ORF_CUDA(cudaMemsetAsync(big, 0, sizeof *big, st));
+        k_fd_biggest<<<296, 256, 0, st>>>(F->vin, F->N(), big);
+        ORF_CUDA(cudaGetLastError());
+    }
+    k_fd_in<<<296, 256, 0, st>>>(F->map(), F->vin, F->f, mode, big);
     ORF_CUDA(cudaGetLastError());
     ORF_TRY(F->solve(F->f, F->x));
-    if (F->S > 1) {
+    if (checked) {
         double eta = 0.0;
         ORF_TRY(F->residual(&eta));
         if (eta > kEtaRefine) ORF_TRY(F->refine());
     }
-    k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode);
+    k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, big);
     ORF_CUDA(cudaGetLastError());
     ORF_TRY(copy_d2h_staged(x, F->vout, bytes, stage, st));
     add_d2h(F->ctx, (int64_t)bytes);

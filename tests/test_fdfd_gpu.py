@@ -193,3 +193,21 @@ def test_fdfd_factorisations_on_several_threads():
     for q in (0, 1):
         assert first[q][0] > 1
         assert all(s == first[q][0] and np.array_equal(E, first[q][1]) for s, E in got[q])
+
+
+@pytest.mark.parametrize("nx,nz", [(120, 40), (33, 150)])
+@pytest.mark.parametrize("power", [-1000, -660, 660, 960])
+def test_fdfd_solution_scales_with_its_source(nx, nz, power):
+    """A source times a power of two gives the field times that power, to the
+    bit: the residual check and its refinement see the same numbers at
+    1e-300 as at 1."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(nx, nz, 3, True)
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    assert o.info()["segments"] > 1
+    s = 2.0 ** power
+    assert np.array_equal(o.solve(J * s), np.ldexp(o.E.real, power) + 1j * np.ldexp(o.E.imag, power))
+    a = o.adjoint(g)
+    assert np.array_equal(o.adjoint(g * s), np.ldexp(a.real, power) + 1j * np.ldexp(a.imag, power))
+    r = oracle_fdfd2D(x, z, eps, lam, J, Npml=npml)
+    assert rel(o.E, r.E) <= TOL
+    o.close()
