@@ -463,8 +463,10 @@ ORF_API int32_t orf_eps3d(orf_ctx* ctx, const double* x, const double* y, const 
  * orf_fdfd2d_factor builds the operator and factors it on the device (block
  * LU along the longer axis, cut into segments eliminated side by side; the
  * shorter axis may hold at most 384 points); each orf_fdfd2d_solve is then
- * sweeps over the segments and the lines between them, with a step of
- * iterative refinement.
+ * sweeps over the segments and the lines between them.  Where there are several
+ * segments a solve checks its residual and is refined while that is above
+ * rounding and falls; if it does not come down, the operator is factored again
+ * as one segment.
  * Complex arrays are interleaved (re, im) pairs of nx*nz entries in
  * column-major order (entry (i, k) at i + nx*k), as MATLAB's interleaved
  * complex API hands them over. */
@@ -488,6 +490,10 @@ ORF_API int32_t orf_fdfd2d_info(const orf_fdfd* f, int32_t* block, int32_t* nblo
 /* segments the lines were to be cut into, and those of the factors (1 where
  * a segment turned out nearly singular by itself, or memory was short) */
 ORF_API int32_t orf_fdfd2d_segments(const orf_fdfd* f, int32_t* planned, int32_t* segments);
+/* residual of the last solve after its refinement, |r| / (|A| |x| + |rhs|) with
+ * the largest entries; -1 before the first one, and where the grid was planned
+ * as one segment (no residual is taken) */
+ORF_API int32_t orf_fdfd2d_residual(const orf_fdfd* f, double* residual);
 ORF_API void    orf_fdfd2d_release(orf_fdfd* f);
 
 #ifdef __cplusplus

@@ -76,6 +76,7 @@ _SIGS = {
     "orf_fdfd2d_solve": (C.c_int32, [C.c_void_p, P(C.c_double), P(C.c_double), C.c_int32]),
     "orf_fdfd2d_info": (C.c_int32, [C.c_void_p, P(C.c_int32), P(C.c_int32), P(C.c_int32)]),
     "orf_fdfd2d_segments": (C.c_int32, [C.c_void_p, P(C.c_int32), P(C.c_int32)]),
+    "orf_fdfd2d_residual": (C.c_int32, [C.c_void_p, P(C.c_double)]),
     "orf_fdfd2d_release": (None, [C.c_void_p]),
     "orf_serve_close": (C.c_int32, [C.c_void_p]),
     "orf_check_violations": (C.c_int32, [P(C.c_uint64), C.c_int32]),

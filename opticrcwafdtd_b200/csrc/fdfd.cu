@@ -28,9 +28,10 @@
 // A segment between two separators is a closed cavity and can be nearly
 // singular where the whole operator is not.  So a factorisation with several
 // segments is tried on one right-hand side: if the residual is not that of a
-// stable solve, the operator is factored again as one segment.  Each solve
-// checks its residual too and takes a step of refinement where it is above
-// rounding.
+// stable solve, the operator is factored again as one segment.  Each solve of an
+// operator in several segments checks its residual too, is refined while that
+// is above rounding and falls, and has the operator factored again as one
+// segment where it does not come down.
 //
 // A solve is a forward and a backward sweep of every segment (for the
 // separators' right-hand side), the separators' two sweeps, and a second pair
@@ -941,6 +942,9 @@ struct orf_fdfd {
     double2 *f = nullptr, *x = nullptr, *r = nullptr, *dx = nullptr, *Y = nullptr, *YT = nullptr, *V = nullptr,
             *Z = nullptr;
     unsigned long long* mx = nullptr;   // largest |r|^2, |x|^2, |f|^2; largest entry of the caller's right-hand side
+    double* h_mx = nullptr;             // the same on the host (pinned)
+    double eta = -1.0;                  // residual of the last solve (-1: none taken)
+    bool singular = false;              // a zero or NaN pivot in the last factorisation
     FdSeg* segs = nullptr;
     int *line = nullptr, *fault = nullptr;
     ~orf_fdfd() {
@@ -948,6 +952,7 @@ struct orf_fdfd {
             cudaStreamSynchronize(ctx->stream);
             ar.release();
         }
+        host_mapped_free(h_mx);
         if (ctx) ctx_release(ctx);
     }
     FdfdDev dev() const { return FdfdDev{m, nb, diag, wc, eb, inv, fault, xrow}; }
@@ -968,18 +973,20 @@ struct orf_fdfd {
         }
         return ORF_OK;
     }
-    // r = f - M x, and its size against rounding: |r| / (|M| |x| + |f|), largest entries
-    int residual(double* eta) {
+    // r = f - M x on the stream; its size reaches the host with it
+    int residual() {
         cudaStream_t st = ctx->stream;
         ORF_CUDA(cudaMemsetAsync(mx, 0, 3 * sizeof *mx, st));
         k_fd_residual<<<296, 256, 0, st>>>(dev(), f, x, r, mx);
         ORF_CUDA(cudaGetLastError());
-        double h[3];
-        ORF_CUDA(cudaMemcpyAsync(h, mx, sizeof h, cudaMemcpyDeviceToHost, st));
-        ORF_CUDA(cudaStreamSynchronize(st));
-        const double den = mnorm * std::sqrt(h[1]) + std::sqrt(h[2]);
-        *eta = h[0] == 0.0 ? 0.0 : std::sqrt(h[0]) / den;
+        ORF_CUDA(cudaMemcpyAsync(h_mx, mx, 4 * sizeof *mx, cudaMemcpyDeviceToHost, st));
         return ORF_OK;
+    }
+    // its size against rounding, |r| / (|M| |x| + |f|) with the largest entries,
+    // once the stream has reached it
+    double eta_now() const {
+        const double den = mnorm * std::sqrt(h_mx[1]) + std::sqrt(h_mx[2]);
+        return h_mx[0] == 0.0 ? 0.0 : std::sqrt(h_mx[0]) / den;
     }
     int refine() {
         ORF_TRY(solve(r, dx));
@@ -987,21 +994,58 @@ struct orf_fdfd {
         ORF_CUDA(cudaGetLastError());
         return ORF_OK;
     }
-    int factor(int nseg, bool* singular);
+    template <class Out>
+    int settle(Out&& out);
+    int factor(int nseg);
+    int refuse_singular() const {
+        if (!singular) return ORF_OK;
+        set_error("fdfd2D: the operator is singular (a zero or NaN pivot in the block elimination)");
+        return ORF_EINVAL;
+    }
 };
 
 namespace {
 // A solve with a residual above kEtaRefine takes a step of refinement: as one
-// segment the residuals are 6e-17 .. 1.3e-16 (error against an exact solve
-// 2e-14 .. 1.4e-13 on grids of 150 x 92 .. 600 x 250), as 15 segments 1e-16 ..
-// 5e-15 (up to 3e-12), and 1e-17 (2e-14 .. 9e-14) after the step.  A
-// factorisation whose trial solve has one above kEtaTrial is done again as
-// one segment.
-constexpr double kEtaRefine = 1e-16, kEtaTrial = 1e-11;
+// segment the residuals are 6e-17 .. 6e-16 (error against an exact solve 2e-14
+// .. 1.4e-13 on grids of 150 x 92 .. 600 x 250), as 15 segments 1e-16 .. 5e-15
+// (up to 3e-12), and 1e-17 .. 2e-16 (2e-14 .. 9e-14) after the step.  Above
+// kEtaAccept it takes up to kRefineSteps in all while the residual falls; if it
+// still ends above, the operator is factored again as one segment (whose solves
+// are refined above kEtaAccept only).  So is a factorisation whose trial solve
+// has a residual above kEtaTrial.
+constexpr double kEtaRefine = 1e-16, kEtaAccept = 1e-15, kEtaTrial = 1e-11;
+constexpr int kRefineSteps = 3;
 }  // namespace
 
+// From the first x of M x = f to the one handed over by out(), which waits for
+// the stream: refined as above, the result under way while the residual of the
+// step before it is taken (out() runs again in the rare case that more is to
+// do).  A right-hand side that is not finite (h_mx[3]: its largest entry) has no
+// residual.
+template <class Out>
+int orf_fdfd::settle(Out&& out) {
+    ORF_TRY(residual());
+    ORF_CUDA(cudaStreamSynchronize(ctx->stream));
+    eta = eta_now();
+    if (!std::isfinite(h_mx[3]) || eta <= (S > 1 ? kEtaRefine : kEtaAccept)) return out();
+    for (int k = 0; k < kRefineSteps; ++k) {
+        const double before = eta;
+        ORF_TRY(refine());
+        ORF_TRY(residual());
+        ORF_TRY(out());
+        eta = eta_now();
+        if (eta <= kEtaAccept) return ORF_OK;
+        if (!(eta < before)) break;   // it falls no more (or is not a number)
+    }
+    if (S == 1) return ORF_OK;
+    ORF_TRY(factor(1));
+    ORF_TRY(refuse_singular());
+    ORF_TRY(solve(f, x));
+    return settle(out);
+}
+
 // Factor the operator as nseg segments.
-int orf_fdfd::factor(int nseg, bool* singular) {
+int orf_fdfd::factor(int nseg) {
     cudaStream_t st = ctx->stream;
     const FdfdDev P = dev();
     const size_t mm = (size_t)m * m;
@@ -1139,7 +1183,7 @@ int orf_fdfd::factor(int nseg, bool* singular) {
     int flt = 0;
     ORF_CUDA(cudaMemcpyAsync(&flt, fault, sizeof(int), cudaMemcpyDeviceToHost, st));
     ORF_CUDA(cudaStreamSynchronize(st));
-    *singular = flt != 0;
+    singular = flt != 0;
     return ORF_OK;
 }
 
@@ -1240,6 +1284,11 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         ar.add(&F->xrow, (size_t)S * kPanel * m);
         return ar.alloc();
     };
+    {
+        void *h = nullptr, *d = nullptr;
+        ORF_TRY(host_mapped_alloc(4 * sizeof(double), &h, &d));
+        F->h_mx = static_cast<double*>(h);
+    }
     int rc = carve();
     if (rc == ORF_ENOMEM_DEVICE && S > 1) {   // one segment needs no memory for separators
         S = 1;
@@ -1255,28 +1304,26 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
     ORF_CUDA(cudaMemcpyAsync(F->sx, hx.data(), nx * sizeof(double2), cudaMemcpyHostToDevice, st));
     ORF_CUDA(cudaMemcpyAsync(F->sz, hz.data(), nz * sizeof(double2), cudaMemcpyHostToDevice, st));
     add_h2d(ctx, (int64_t)((3 * N + nx + nz) * sizeof(double2)));
-    bool singular = false;
-    rc = F->factor(S, &singular);
+    rc = F->factor(S);
     if (rc == ORF_ENOMEM_DEVICE && S > 1) {   // (the separators' blocks; every other error is the caller's to see)
         S = 1;
-        rc = F->factor(S, &singular);
+        rc = F->factor(S);
     }
     ORF_TRY(rc);
     if (S > 1) {
         // a segment that is nearly singular by itself shows in a trial solve
-        double eta = 0.0;
-        if (!singular) {
+        double trial = 0.0;
+        if (!F->singular) {
             k_fd_probe<<<296, 256, 0, st>>>(F->f, N);
             ORF_CUDA(cudaGetLastError());
             ORF_TRY(F->solve(F->f, F->x));
-            ORF_TRY(F->residual(&eta));
+            ORF_TRY(F->residual());
+            ORF_CUDA(cudaStreamSynchronize(st));
+            trial = F->eta_now();
         }
-        if (singular || !(eta <= kEtaTrial)) ORF_TRY(F->factor(1, &singular));
+        if (F->singular || !(trial <= kEtaTrial)) ORF_TRY(F->factor(1));
     }
-    if (singular) {
-        set_error("fdfd2D: the operator is singular (a zero or NaN pivot in the block elimination)");
-        return ORF_EINVAL;
-    }
+    ORF_TRY(F->refuse_singular());
     *out = F.release();
     return ORF_OK;
 }
@@ -1286,6 +1333,7 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
         set_error("fdfd handle, rhs and x are required");
         return ORF_EINVAL;
     }
+    ORF_TRY(F->refuse_singular());   // (found by an earlier solve)
     ORF_ON_DEVICE(F->ctx->device);
     const size_t bytes = F->N() * sizeof(double2);
     const int mode = transpose ? 1 : 0;
@@ -1302,7 +1350,8 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
     } rel{stage, st};
     ORF_TRY(copy_h2d_staged(F->vin, rhs, bytes, stage, st));
     add_h2d(F->ctx, (int64_t)bytes);
-    const bool checked = F->S > 1;   // (as one segment: no residual is taken, nothing to scale for)
+    // (planned as one segment: no residual is taken, nothing to scale for)
+    const bool checked = F->planned > 1;
     unsigned long long* big = checked ? F->mx + 3 : nullptr;
     if (checked) {
         ORF_CUDA(cudaMemsetAsync(big, 0, sizeof *big, st));
@@ -1311,15 +1360,13 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
     }
     k_fd_in<<<296, 256, 0, st>>>(F->map(), F->vin, F->f, mode, big);
     ORF_CUDA(cudaGetLastError());
+    auto result = [&]() -> int {   // of the solve so far, into the caller's array
+        k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, big);
+        ORF_CUDA(cudaGetLastError());
+        return copy_d2h_staged(x, F->vout, bytes, stage, st);
+    };
     ORF_TRY(F->solve(F->f, F->x));
-    if (checked) {
-        double eta = 0.0;
-        ORF_TRY(F->residual(&eta));
-        if (eta > kEtaRefine) ORF_TRY(F->refine());
-    }
-    k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, big);
-    ORF_CUDA(cudaGetLastError());
-    ORF_TRY(copy_d2h_staged(x, F->vout, bytes, stage, st));
+    ORF_TRY(checked ? F->settle(result) : result());
     add_d2h(F->ctx, (int64_t)bytes);
     return ORF_OK;
 }
@@ -1348,5 +1395,14 @@ extern "C" int32_t orf_fdfd2d_segments(const orf_fdfd* F, int32_t* planned, int3
     }
     if (planned) *planned = F->planned;
     if (segments) *segments = F->S;
+    return ORF_OK;
+}
+
+extern "C" int32_t orf_fdfd2d_residual(const orf_fdfd* F, double* residual) {
+    if (!F || !residual) {
+        set_error("fdfd handle and residual are required");
+        return ORF_EINVAL;
+    }
+    *residual = F->eta;
     return ORF_OK;
 }

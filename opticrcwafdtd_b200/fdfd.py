@@ -16,6 +16,7 @@ indices as in the reference's calls, > 0 toward +x / +z).
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 
 import numpy as np
 
@@ -75,7 +76,12 @@ class FDFD2D:
         planned, segs = C.c_int32(), C.c_int32()
         _lib.check(self.lib.orf_fdfd2d_segments(self.handle, C.byref(planned), C.byref(segs)), "fdfd2D info")
         return {"block": m.value, "blocks": nb.value, "cluster": cl.value, "planned_segments": planned.value,
-                "segments": segs.value}
+                "segments": segs.value, "residual": self._residual()}
+
+    def _residual(self) -> float:
+        r = C.c_double()
+        _lib.check(self.lib.orf_fdfd2d_residual(self.handle, C.byref(r)), "fdfd2D residual")
+        return r.value
 
     def _run(self, v, transpose: int) -> np.ndarray:
         if self.handle is None:
@@ -85,6 +91,9 @@ class FDFD2D:
         _lib.check(self.lib.orf_fdfd2d_solve(self.handle, rhs.view(np.float64).ctypes.data_as(_abi.c_double_p),
                                              out.view(np.float64).ctypes.data_as(_abi.c_double_p), transpose),
                    "fdfd2D solve")
+        if self._residual() > 1e-12:
+            warnings.warn("fdfd2D: the operator is nearly singular; the solution's residual is "
+                          f"{self._residual():.1e}", RuntimeWarning, stacklevel=3)
         return out.reshape((self.nx, self.nz), order="F")
 
     def solve(self, J2) -> np.ndarray:

@@ -211,3 +211,31 @@ def test_fdfd_solution_scales_with_its_source(nx, nz, power):
     r = oracle_fdfd2D(x, z, eps, lam, J, Npml=npml)
     assert rel(o.E, r.E) <= TOL
     o.close()
+
+
+@pytest.mark.parametrize("detuning", [0.0, 1e-8, 1e-5, 1e-4, 5e-4, 1e-3, 3e-3, 1e-2])
+def test_fdfd_segments_near_resonance(detuning):
+    """The cavity of test_fdfd_segment_in_resonance moved off its segments'
+    resonance by a little: trial residuals from far above what is refused to
+    that of an ordinary operator.  Sources all over, on one cell and in the
+    shape of a segment's mode: the residual is that of a stable solve however
+    many segments the factors keep, and the field and adjoint the oracle's."""
+    nx, nz, d, lam = 41, 6, 0.03, 1.3
+    ev = 4 / d ** 2 * (np.sin(np.pi / (2 * 6)) ** 2 + np.sin(np.pi / (2 * 7)) ** 2)
+    eps = np.full((nx, nz), ev * (1 + detuning) / (2 * np.pi / lam) ** 2)
+    eps[:5] *= 1.3
+    eps[36:] *= 1.5
+    x, z = np.arange(nx) * d, np.arange(nz) * d
+    rng = np.random.default_rng(6)
+    every = rng.standard_normal((nx, nz)) + 1j * rng.standard_normal((nx, nz))
+    cell, mode = np.zeros((2, nx, nz))
+    cell[14, 2] = 1.0
+    mode[12:17] = np.outer(np.sin(np.pi * np.arange(1, 6) / 6), np.sin(np.pi * np.arange(1, 7) / 7))
+    o = orf.fdfd2D(x, z, eps, lam, every, Npml=(0, 0))
+    r = oracle_fdfd2D(x, z, eps, lam, every, Npml=(0, 0))
+    assert o.info()["planned_segments"] == 7
+    for J in (every, cell, mode):
+        for a, b in ((o.solve, r.solve), (o.adjoint, r.adjoint)):
+            assert rel(a(J), b(J)) <= TOL
+            assert 0.0 <= o.info()["residual"] <= 1e-15
+    o.close()
