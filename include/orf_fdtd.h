@@ -260,6 +260,12 @@ typedef struct orf_tile3d {
 ORF_API int32_t orf_plan3d(const orf_sim3d* sim, orf_tile3d* tiles, int32_t cap, int32_t* n_interior,
                            int32_t* n_cpml);
 
+/* The same for run `which` of n_sims runs whose launches are shared (a server's
+ * jobs of one precision and index width): the segments are cut for all of them
+ * together.  orf_plan3d is the case of one run. */
+ORF_API int32_t orf_plan3d_group(const orf_sim3d* sims, int32_t n_sims, int32_t which, orf_tile3d* tiles,
+                                 int32_t cap, int32_t* n_interior, int32_t* n_cpml);
+
 /* No counterpart in the reference.  The checked build of this library
  * (lib/liborf_fdtd_check.so, compiled with ORF_CHECK) tests every global
  * access of the 2D step kernels against its buffer and every stored cell

@@ -354,9 +354,25 @@ int32_t orf_plan2d(const orf_sim2d* sim, const orf_tuning* tuning, orf_tile2d* t
 }
 
 int32_t orf_plan3d(const orf_sim3d* sim, orf_tile3d* tiles, int32_t cap, int32_t* n_interior, int32_t* n_cpml) {
-    ORF_TRY(validate3d(sim));
+    return orf_plan3d_group(sim, 1, 0, tiles, cap, n_interior, n_cpml);
+}
+
+int32_t orf_plan3d_group(const orf_sim3d* sims, int32_t n_sims, int32_t which, orf_tile3d* tiles, int32_t cap,
+                         int32_t* n_interior, int32_t* n_cpml) {
+    if (!sims || n_sims < 1 || which < 0 || which >= n_sims) {
+        set_error("orf_plan3d_group: which must name one of the sims");
+        return ORF_EINVAL;
+    }
+    std::vector<Layout3D> lays(n_sims);
+    std::vector<const Layout3D*> runs;
+    for (int q = 0; q < n_sims; ++q) {
+        ORF_TRY(validate3d(sims + q));
+        lays[q] = layout3d(sims + q);
+        runs.push_back(&lays[q]);
+    }
+    const orf_sim3d* sim = sims + which;
     std::vector<Tile3D> ti, tp;
-    plan3d(sim, ti, tp);
+    cut3d(lays[which], seg_lengths(runs, sim->precision == ORF_DOUBLE, orf_ctx{}.sm_count), 0, ti, tp);
     if (n_interior) *n_interior = (int32_t)ti.size();
     if (n_cpml) *n_cpml = (int32_t)tp.size();
     const size_t n = ti.size() + tp.size();

@@ -173,24 +173,27 @@ struct Group2D : Group {
     }
 };
 
-// 3D members share precision and index width (zc is the z-segment length,
-// the same for every job).
+// 3D members share precision and index width.  Their tiles are cut anew for the
+// group (seg_lengths): the short segments that let one small run fill the SMs are
+// nearly twice the work once many runs do, each start being paid by an SM that has
+// other segments to march.  22 x 22 x 171 periodic FP32 runs served together, us
+// per step of all, cut each by itself / for the group / into the longest segments:
+// 4 runs 25 / 22 / 52, 16 runs 60 / 52 / 105, 64 runs 224 / 170 / 170.  Over 154
+// sets of 2 to 64 runs of six grids in both precisions the group's cut takes 0.92
+// times the better of the other two (at worst 1.12).  It changes no bit.
 template <class R>
 struct Group3D : Group {
     std::vector<Job3D<R>*> jobs;
-    int zc = 4, idxw = 1;
+    int idxw = 1;
     Inst3D<R>* d_insts = nullptr;
     Tile3D *d_tiles = nullptr, *d_tiles_pml = nullptr;
     int nt = 0, ntp = 0;
     SideStream side;   // CPML tiles next to the interior tiles
     int64_t all_cells = 0;
 
-    static bool compatible(const Job3D<R>* a, const Job3D<R>* b) { return a->zc == b->zc && a->idxw == b->idxw; }
+    static bool compatible(const Job3D<R>* a, const Job3D<R>* b) { return a->idxw == b->idxw; }
     void add(Job3D<R>* j) {
-        if (jobs.empty()) {
-            zc = j->zc;
-            idxw = j->idxw;
-        }
+        if (jobs.empty()) idxw = j->idxw;
         jobs.push_back(j);
         dirty = true;
     }
@@ -212,17 +215,12 @@ struct Group3D : Group {
         items.clear();
         states.clear();
         all_cells = 0;
+        std::vector<const Layout3D*> lays;
+        for (auto* j : jobs) lays.push_back(&j->lay);
+        const SegLen3D len = seg_lengths(lays, sizeof(R) == 8, ctx->sm_count);
         for (auto* j : jobs) {
-            const int id = (int)insts.size();
+            cut3d(j->lay, len, (int)insts.size(), tl, tp);
             insts.push_back(j->h);
-            for (Tile3D t : j->tiles) {
-                t.inst = id;
-                tl.push_back(t);
-            }
-            for (Tile3D t : j->tiles_pml) {
-                t.inst = id;
-                tp.push_back(t);
-            }
             all_cells += j->cells();
             add_streams(j->host_streams, j->nL, j->d_st);
         }

@@ -121,108 +121,154 @@ int Job3D<R>::encode_tmap3(CUtensorMap* m, CUtensorMapDataType t, const void* ba
     return ORF_OK;
 }
 
-// Segment lengths of a 3D run.  A CTA marches its segment plane by plane, a
-// serial chain: 5 us + 0.92 us a plane (CPML: 3.6 + 3.2) while the SM has little
-// else to do; a full SM spends 0.48 us (CPML 1.09) on a plane, and a segment
-// costs about five planes' worth of start.  One launch then takes about the
-// longest segment's chain plus the work shared by the SMs: short segments win
-// while the grid leaves SMs idle, long ones once it fills them.  Both lengths
-// are chosen to minimise that estimate, within kSeg3 (the constants fitted to
-// 120 timed steps of ten grids and twelve pairs of lengths on a B200, rms
-// error 15 %; the choice within 13 % of the best of the twelve on each).
-// Per step, against segments of up to kSeg3 planes: 22 x 22 x 171 periodic FP32
-// 64 -> 13 us, 201 x 93 x 77 with CPML on all sides 239 -> 85 us, 200 x 160 x
-// 141 FP64 244 -> 202 us; 320 x 320 x 200 and larger keep the long segments
-// (with shorter ones 379 -> 402 us).
+// Segment lengths.  A CTA marches its segment plane by plane, a serial chain, and
+// pays for a segment's start: short segments win while SMs would idle, long ones
+// once there are CTAs enough.  The lengths for the planes away from and at the z
+// slabs are the pair with the least estimated time of a step.
 namespace {
-struct SegPlan {
-    int in, pml;   // planes of a segment at most, away from and at the z slabs
+constexpr int kLen[] = {60, 40, 30, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2}, kLens = (int)(sizeof(kLen) / sizeof(int));
+
+// CTAs of one kind of tile (interior, CPML), by length of their segments' zone
+struct SegLoad {
+    double n = 0.0, planes = 0.0, longest = 0.0;   // CTAs, their planes, planes of the longest segment
+    void add(double ctas, double len) {
+        n += ctas;
+        planes += ctas * len;
+        longest = std::max(longest, len);
+    }
+    SegLoad operator+(const SegLoad& o) const { return {n + o.n, planes + o.planes, std::max(longest, o.longest)}; }
 };
-SegPlan seg_lengths(int cols_in, int cols_pml, const std::vector<std::pair<int, bool>>& zones) {
-    constexpr double kSm = 148.0, kStart = 5.1;
-    constexpr double kFixed[2] = {5.0, 3.65}, kAlone[2] = {0.92, 3.24}, kShared[2] = {0.475, 1.09};   // in, pml
-    static const int kLen[] = {60, 40, 30, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2};
-    SegPlan best{kSeg3, kSeg3};
-    double best_t = -1.0;
-    for (int li : kLen)
-        for (int lp : kLen) {
-            double chain = 0.0, work = 0.0;
-            for (auto [planes, pml] : zones) {
-                const int c = (planes + (pml ? lp : li) - 1) / (pml ? lp : li);
+
+// A step of one run: 5 us + 0.92 us a plane of the longest segment (CPML: 3.6 +
+// 3.2) while the SM has little else to do, plus the work shared by the SMs, 0.48
+// us (CPML 1.09) a plane and about five planes' worth of start per segment (the
+// constants fitted to 120 timed steps of ten grids and twelve pairs of lengths
+// on a B200, rms error 15 %; the choice within 13 % of the best of the twelve on
+// each).  Per step, against segments of up to kSeg3 planes: 22 x 22 x 171
+// periodic FP32 64 -> 13 us, 201 x 93 x 77 with CPML on all sides 239 -> 85 us,
+// 200 x 160 x 141 FP64 244 -> 202 us; 320 x 320 x 200 and larger keep the long
+// segments (with shorter ones 379 -> 402 us).
+double step_alone(const SegLoad& in, const SegLoad& pml, int sms) {
+    const double chain = std::max(in.n > 0 ? 5.0 + 0.92 * in.longest : 0.0, pml.n > 0 ? 3.65 + 3.24 * pml.longest : 0.0);
+    return chain + ((in.planes + 5.1 * in.n) * 0.475 + (pml.planes + 5.1 * pml.n) * 1.09) / sms;
+}
+
+// A step of a group of runs.  A plane costs a CTA more the more CTAs its SM holds
+// (at most 4 FP32 interior ones, 3 of any other kind).  An SM that holds FP32
+// interior tiles takes no CPML tiles beside them (the kernels split shared memory
+// differently): those wait, unless SMs without interior tiles hold them all.
+// Fitted to 3600 timed steps, 1 to 64 equal runs of seven grids in both precisions
+// with 66 pairs of lengths: rms error 6 %.  (step_alone adds the whole of the
+// shared work to the chain: right within 15 % for one run, but between a few runs
+// and many it keeps segments too long or too short.)
+template <bool F64>
+double step_group(const SegLoad& in, const SegLoad& pml, int sms) {
+    struct K {
+        double fixed, plane, per_cta, start;   // us; us a plane by itself, more per CTA on the SM; planes
+        int cap;                               // CTAs an SM holds
+    };
+    constexpr K kIn = F64 ? K{0.0, 0.79, 0.57, 2.9, 3} : K{3.0, 0.565, 0.355, 3.0, 4};
+    constexpr K kPml = F64 ? K{0.0, 2.5, 1.23, 1.0, 3} : K{0.0, 2.35, 0.66, 2.0, 3};
+    constexpr double kTail = F64 ? 0.40 : 0.43, kHidden = F64 ? 0.18 : 0.27, kShare = 0.15;
+    auto alone = [sms](const K& k, const SegLoad& l) {
+        if (l.n <= 0.0) return 0.0;
+        const double r = std::ceil(l.n / sms);
+        if (r <= k.cap) return k.fixed + (l.longest + k.start) * (k.plane + r * k.per_cta);
+        const double full = k.plane + k.cap * k.per_cta;   // waves, and a last one partly filled
+        return k.fixed + ((l.planes + k.start * l.n) / ((double)sms * k.cap) + kTail * l.longest) * full;
+    };
+    const double a = alone(kIn, in), b = alone(kPml, pml), least = std::min(a, b);
+    if (F64 && in.n + pml.n <= 3.0 * sms) return std::max(a, b) + kShare * least;
+    if (!F64 && pml.n <= 3.0 * (sms - in.n)) return std::max(a, b);
+    return a + b - kHidden * least;
+}
+}  // namespace
+
+SegLen3D seg_lengths(const std::vector<const Layout3D*>& runs, bool fp64, int sm_count) {
+    SegLoad in[2][kLens], pml[2][kLens];   // by zone: away from the z slabs, at them
+    for (const Layout3D* r : runs)
+        for (auto [planes, at_slab] : r->zones)
+            for (int q = 0; q < kLens; ++q) {
+                const int c = (planes + kLen[q] - 1) / kLen[q], nin = at_slab ? 0 : r->cols_in;
                 const double len = (double)planes / c;
-                const int nin = pml ? 0 : cols_in, npml = cols_in + cols_pml - nin;
-                if (nin) chain = std::max(chain, kFixed[0] + len * kAlone[0]);
-                if (npml) chain = std::max(chain, kFixed[1] + len * kAlone[1]);
-                work += c * (len + kStart) * (nin * kShared[0] + npml * kShared[1]);
+                if (nin > 0) in[at_slab][q].add((double)c * nin, len);
+                const int npml = r->cols_in + r->cols_pml - nin;
+                if (npml > 0) pml[at_slab][q].add((double)c * npml, len);
             }
-            const double t = chain + work / kSm;
+    const auto step = runs.size() == 1 ? step_alone : fp64 ? step_group<true> : step_group<false>;
+    SegLen3D best{kSeg3, kSeg3};
+    double best_t = -1.0;
+    for (int li = 0; li < kLens; ++li)
+        for (int lp = 0; lp < kLens; ++lp) {
+            const double t = step(in[0][li] + in[1][lp], pml[0][li] + pml[1][lp], std::max(1, sm_count));
             if (best_t < 0.0 || t < 0.99 * best_t) {   // the longer lengths come first
                 best_t = t;
-                best = SegPlan{li, lp};
+                best = SegLen3D{kLen[li], kLen[lp]};
             }
         }
     return best;
 }
-}  // namespace
 
-// Host-only plan of a 3D run's tiles: kTile3X x kTile3Y columns, a segment
-// of up to kSeg3 planes each (seg_lengths); a tile takes the CPML
-// instantiation if any cell it updates or recomputes (one halo cell in x and
-// y, the plane below the segment) lies within one cell of an absorbing slab
-// along any axis.  z segments never mix planes near a z slab with planes away
-// from it, so only the planes that need CPML code run it.  Needs no device;
-// orf_plan3d exposes it for checks of the tiling.
-void plan3d(const orf_sim3d* s, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml, bool zlo, bool zhi) {
+bool Layout3D::near_pml(int q, int lo, int hi) const {
+    if (np[q] <= 0) return false;
+    const bool at_lo = q != 2 || zlo, at_hi = q != 2 || zhi;
+    return (at_lo && lo < np[q] + 1) || (at_hi && hi > n[q] - np[q] - 2);
+}
+
+Layout3D layout3d(const orf_sim3d* s, bool zlo, bool zhi) {
+    Layout3D a;
     const int n[3] = {s->nx, s->ny, s->nz};
-    bool per[3];
-    for (int q = 0; q < 3; ++q) per[q] = s->periodic[q] != 0;
-    tiles.clear();
-    tiles_pml.clear();
-    auto near_pml = [&](int q, int lo, int hi) {   // cells [lo, hi) along axis q
-        const int np = per[q] ? 0 : s->npml[q];
-        if (np <= 0) return false;
-        const bool at_lo = q != 2 || zlo, at_hi = q != 2 || zhi;
-        return (at_lo && lo < np + 1) || (at_hi && hi > n[q] - np - 2);
-    };
-    // the columns near an x / y slab, and the runs of planes near a z slab or
-    // away from both
-    int cols_in = 0, cols_pml = 0;
+    for (int q = 0; q < 3; ++q) {
+        a.n[q] = n[q];
+        a.np[q] = s->periodic[q] ? 0 : s->npml[q];
+    }
+    a.zlo = zlo;
+    a.zhi = zhi;
     for (int j0 = 0; j0 < n[1]; j0 += kTile3Y)
         for (int i0 = 0; i0 < n[0]; i0 += kTile3X) {
-            const bool pm = near_pml(0, i0 - 1, std::min(i0 + kTile3X, n[0]) + 1) ||
-                            near_pml(1, j0 - 1, std::min(j0 + kTile3Y, n[1]) + 1);
-            ++(pm ? cols_pml : cols_in);
+            const bool pm = a.near_pml(0, i0 - 1, std::min(i0 + kTile3X, n[0]) + 1) ||
+                            a.near_pml(1, j0 - 1, std::min(j0 + kTile3Y, n[1]) + 1);
+            ++(pm ? a.cols_pml : a.cols_in);
         }
-    std::vector<std::pair<int, bool>> zones;
     for (int k0 = 0; k0 < n[2];) {
-        const bool pz0 = near_pml(2, k0 - 1, k0 + 2);
+        const bool pz0 = a.near_pml(2, k0 - 1, k0 + 2);
         int k1 = k0 + 1;
-        while (k1 < n[2] && near_pml(2, k1 - 1, k1 + 2) == pz0) ++k1;
-        zones.push_back({k1 - k0, pz0});
+        while (k1 < n[2] && a.near_pml(2, k1 - 1, k1 + 2) == pz0) ++k1;
+        a.zones.push_back({k1 - k0, pz0});
         k0 = k1;
     }
-    const SegPlan len = seg_lengths(cols_in, cols_pml, zones);
+    return a;
+}
+
+// Tiles of a 3D run: kTile3X x kTile3Y columns, a segment of up to kSeg3 planes
+// each (seg_lengths); a tile takes the CPML instantiation if any cell it updates
+// or recomputes (one halo cell in x and y, the plane below the segment) lies
+// within one cell of an absorbing slab along any axis.  z segments never mix
+// planes near a z slab with planes away from it, so only the planes that need
+// CPML code run it.  Needs no device; orf_plan3d and orf_plan3d_group expose it
+// for checks of the tiling.
+void cut3d(const Layout3D& a, SegLen3D len, int inst, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml) {
     std::vector<std::pair<int, int>> segs;
     int z0 = 0;
-    for (auto [planes, pz0] : zones) {   // equal segments
+    for (auto [planes, pz0] : a.zones) {   // equal segments
         const int c = (planes + (pz0 ? len.pml : len.in) - 1) / (pz0 ? len.pml : len.in);
         for (int q = 0; q < c; ++q)
             segs.push_back({z0 + (int)((int64_t)planes * q / c), z0 + (int)((int64_t)planes * (q + 1) / c)});
         z0 += planes;
     }
     for (auto [k0, k1] : segs)
-        for (int j0 = 0; j0 < n[1]; j0 += kTile3Y)
-            for (int i0 = 0; i0 < n[0]; i0 += kTile3X) {
+        for (int j0 = 0; j0 < a.n[1]; j0 += kTile3Y)
+            for (int i0 = 0; i0 < a.n[0]; i0 += kTile3X) {
                 Tile3D t;
-                t.inst = 0;
+                t.inst = inst;
                 t.i0 = i0;
                 t.j0 = j0;
-                t.tw = (short)std::min(kTile3X, n[0] - i0);
-                t.th = (short)std::min(kTile3Y, n[1] - j0);
+                t.tw = (short)std::min(kTile3X, a.n[0] - i0);
+                t.th = (short)std::min(kTile3Y, a.n[1] - j0);
                 t.k0 = k0;
                 t.k1 = k1;
-                const bool pm = near_pml(0, t.i0 - 1, t.i0 + t.tw + 1) || near_pml(1, t.j0 - 1, t.j0 + t.th + 1) ||
-                                near_pml(2, t.k0 - 1, t.k1 + 1);
+                const bool pm = a.near_pml(0, t.i0 - 1, t.i0 + t.tw + 1) ||
+                                a.near_pml(1, t.j0 - 1, t.j0 + t.th + 1) || a.near_pml(2, t.k0 - 1, t.k1 + 1);
                 (pm ? tiles_pml : tiles).push_back(t);
             }
 }
@@ -380,11 +426,13 @@ int Job3D<R>::create(const orf_sim3d* s) {
         pairs.push_back({4 * m, 4 * m + 3, 4 * m + 1, 4 * m + 2, m, nM, 0.5 * d * d});
     npairs = (int)pairs.size();
 
-    // ---- tiles (plan3d)
+    // ---- tiles
     // a z slab's ends that border other slabs carry no CPML: their planes are
     // interior tiles (the psi planes of the layout there stay unused)
-    plan3d(s, tiles, tiles_pml, !slab || z_off == 0, !slab || z_off + n[2] == nz_glob);
-    zc = kSeg3;
+    lay = layout3d(s, !slab || z_off == 0, !slab || z_off + n[2] == nz_glob);
+    tiles.clear();
+    tiles_pml.clear();
+    cut3d(lay, seg_lengths({&lay}, sizeof(R) == 8, ctx->sm_count), 0, tiles, tiles_pml);
 
     // ---- device arena
     // fields and psi ping-pong: a step reads buffer par and writes par^1

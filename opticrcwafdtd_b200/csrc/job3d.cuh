@@ -6,17 +6,32 @@
 
 namespace orf {
 
-// Host-only tile plan of a 3D run (job3d.cu): interior tiles and CPML tiles.
+// What the tiles of a 3D run are cut from: its kTile3X x kTile3Y columns, those
+// near an x / y CPML slab and the others, and its runs of z planes near a z slab
+// (true) or away from both.
+struct Layout3D {
+    int n[3] = {0, 0, 0}, np[3] = {0, 0, 0};   // np: CPML planes per end, 0 on a periodic axis
+    bool zlo = true, zhi = true;
+    int cols_in = 0, cols_pml = 0;
+    std::vector<std::pair<int, bool>> zones;
+    bool near_pml(int q, int lo, int hi) const;   // cells [lo, hi) along axis q
+};
+struct SegLen3D {
+    int in, pml;   // planes of a segment at most, away from and at the z slabs
+};
 // zlo / zhi: the low / high z end has its CPML layer (false: the end of a z
 // slab that borders another slab, whose planes run as interior tiles)
-void plan3d(const orf_sim3d* s, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml, bool zlo = true,
-            bool zhi = true);
+Layout3D layout3d(const orf_sim3d* s, bool zlo = true, bool zhi = true);
+// the segment lengths of runs that share their launches (job3d.cu)
+SegLen3D seg_lengths(const std::vector<const Layout3D*>& runs, bool fp64, int sm_count);
+// append the run's interior and CPML tiles, as instance inst
+void cut3d(const Layout3D& lay, SegLen3D len, int inst, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml);
 
 template <class R>
 struct Job3D : orf_job {
     int n[3] = {0, 0, 0};
     bool per[3] = {false, false, false};
-    int pitch = 0, nM = 0, nL = 0, idxw = 1, zc = 4;
+    int pitch = 0, nM = 0, nL = 0, idxw = 1;
     double d = 0, Cc = 0, S = 0, src_end = 0, shutoff = 0;
     int64_t nmax = 0, nsrc = 0, enq_steps = 0;
     // z slab of a larger grid (orf_job3d_create_slab): global index of local
@@ -32,7 +47,8 @@ struct Job3D : orf_job {
     Inst3D<R>* d_inst = nullptr;
     JobState* d_st = nullptr;
     JobState** d_states = nullptr;
-    std::vector<Tile3D> tiles, tiles_pml;   // interior / CPML tiles
+    Layout3D lay;
+    std::vector<Tile3D> tiles, tiles_pml;   // interior / CPML tiles of the run by itself
     Tile3D* d_tiles = nullptr;
     Tile3D* d_tiles_pml = nullptr;
     DftStream* d_streams = nullptr;

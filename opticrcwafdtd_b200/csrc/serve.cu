@@ -224,7 +224,7 @@ struct orf_server {
             *fits = !((st == ORF_ETOOLARGE && j->need > left) || st == ORF_ENOMEM_DEVICE);
             return st;
         }
-        const int64_t key = 3 | (int64_t)(sizeof(R) == 8) << 2 | (int64_t)j->idxw << 8 | (int64_t)j->zc << 16 |
+        const int64_t key = 3 | (int64_t)(sizeof(R) == 8) << 2 | (int64_t)j->idxw << 8 |
                             size_class(j->cells()) << 24;
         Group* g = group_for(key);
         if (!g) {

@@ -147,17 +147,19 @@ def plan2d(sim, tsteps: int = 0, variant: int = 0) -> dict:
     return {"tsteps": T.value, "variant": v.value, "n_interior": ni.value, "n_frame": nf.value, "tiles": tiles}
 
 
-def plan3d(sim) -> dict:
-    """The tiles a 3D run of sim would use (orf_plan3d; host only):
+def plan3d(sim, beside=()) -> dict:
+    """The tiles a 3D run of sim would use (orf_plan3d; host only), by itself
+    or in a group with the sims beside it (orf_plan3d_group):
     {"n_interior", "n_cpml", "tiles"}, tiles as a dict of int arrays (kind,
     i0, j0, tw, th, k0, k1, tma, tma_x, tma_index_x), interior tiles first."""
     lib = _lib.load()
-    m = _abi.marshal_sim3d(sim)
+    ms = [_abi.marshal_sim3d(s) for s in (sim, *beside)]
+    sims = (_abi.OrfSim3D * len(ms))(*[m.struct for m in ms])
     ni, nc = C.c_int32(), C.c_int32()
-    _lib.check(lib.orf_plan3d(C.byref(m.struct), None, 0, C.byref(ni), C.byref(nc)), "orf_plan3d")
+    _lib.check(lib.orf_plan3d_group(sims, len(ms), 0, None, 0, C.byref(ni), C.byref(nc)), "orf_plan3d")
     n = ni.value + nc.value
     arr = (_abi.OrfTile3D * max(1, n))()
-    _lib.check(lib.orf_plan3d(C.byref(m.struct), arr, n, C.byref(ni), C.byref(nc)), "orf_plan3d")
+    _lib.check(lib.orf_plan3d_group(sims, len(ms), 0, arr, n, C.byref(ni), C.byref(nc)), "orf_plan3d")
     tiles = {k: np.array([getattr(arr[q], k) for q in range(n)], dtype=np.int64) for k, _ in _abi.OrfTile3D._fields_}
     return {"n_interior": ni.value, "n_cpml": nc.value, "tiles": tiles}
 

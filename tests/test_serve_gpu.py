@@ -176,3 +176,24 @@ def test_preemption_frees_memory_for_the_queue():
     with pytest.raises(orf.OrfError):
         srv.preempt(10 ** 6)
     srv.close()
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_served_3d_set_is_recut_bitwise(precision):
+    """Nine 3D runs of two kinds, joining and leaving a group at different
+    times: its tiles are cut anew for the members of each moment (a few short
+    segments each for one run, longer ones for many), and every run stays
+    bitwise the run by itself."""
+    sims = [cases.box3d_sim(n=(36 + 4 * q, 30, 64 + q), per=(q % 2 == 0, q % 3 == 0, False), steps=120 + 60 * q,
+                            seed=80 + q, precision=precision) for q in range(9)]
+    alone = [orf.fdtd3D(s) for s in sims]
+    srv = orf.Server(macro_steps=50)
+    t = [srv.submit(s, dims=3) for s in sims[:2]]
+    srv.step()
+    t += [srv.submit(s, dims=3) for s in sims[2:6]]
+    srv.step()
+    t += [srv.submit(s, dims=3) for s in sims[6:]]
+    srv.drain()
+    for ticket, a in zip(t, alone):
+        _bitwise3d(srv.result(ticket), a)
+    srv.close()

@@ -217,3 +217,34 @@ def test_3d_segments_fit_the_grid(n, npml, per, longest):
     first = (t["i0"] == 0) & (t["j0"] == 0)
     inner = first & (t["k0"] > npml[2] + 1) & (t["k1"] < n[2] - npml[2] - 2)
     assert np.ptp(length[inner]) <= 1
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("n,npml,per", [((22, 22, 171), (0, 0, 12), (True, True, False)),
+                                        ((64, 40, 77), (8, 8, 8), (False, False, False))])
+def test_3d_runs_together_are_cut_into_longer_segments(n, npml, per, precision):
+    """A run by itself takes short segments to fill the SMs; beside 63 like it
+    the starts of short segments are work that nobody waits for, and the same
+    run is cut into fewer.  Its tiles cover its cells once either way."""
+    from opticrcwafdtd_b200.fdtd import plan3d
+    sim = dict(_sim3d(n, npml, per), precision=precision)
+    tiles = {}
+    for beside in (0, 3, 63):
+        t = tiles[beside] = plan3d(sim, [sim] * beside)["tiles"]
+        cover = np.zeros(n, dtype=np.int32)
+        for q in range(t["kind"].size):
+            cover[t["i0"][q]:t["i0"][q] + t["tw"][q], t["j0"][q]:t["j0"][q] + t["th"][q], t["k0"][q]:t["k1"][q]] += 1
+            assert 1 <= t["k1"][q] - t["k0"][q] <= 60
+        assert np.all(cover == 1)
+    starts = {b: np.unique(t["k0"]).size for b, t in tiles.items()}
+    assert starts[0] >= starts[3] > starts[63]
+    assert starts[63] <= starts[0] / 2
+
+
+def test_3d_plan_beside_a_large_run():
+    """A small run beside a grid that fills the SMs by itself is cut long."""
+    from opticrcwafdtd_b200.fdtd import plan3d
+    cell = _sim3d((22, 22, 171), (0, 0, 12), (True, True, False))
+    lattice = _sim3d((320, 320, 200), (0, 0, 20), (True, True, False))
+    t = plan3d(cell, [lattice])["tiles"]
+    assert np.max(t["k1"] - t["k0"]) >= 30
