@@ -71,3 +71,15 @@ def test_wait_injection_rejects_negative_limit():
     with pytest.raises(_abi.OrfError):
         ctx.set_wait_injection(stall_plane=-1, wait_ns=-5)
     ctx.close()
+
+
+@pytest.mark.parametrize("plane", [0, 20, 59, 2 ** 31 - 1])
+def test_stalled_plane_beyond_a_short_segment_times_out_too(plane):
+    """The segments of a small grid are shorter than the hook's plane: their
+    last plane stalls, so that the hook never passes in silence."""
+    ctx = Context(0)
+    ctx.set_wait_injection(stall_plane=plane, wait_ns=2_000_000)
+    with pytest.raises(_abi.OrfError) as ei:
+        _run(ctx, _sim())
+    assert ei.value.identifier == "orf:deviceTimeout"
+    ctx.close()
