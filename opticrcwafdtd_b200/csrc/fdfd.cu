@@ -807,6 +807,7 @@ __global__ void k_fd_add(double2* __restrict__ x, const double2* __restrict__ dx
         x[o] = cadd(x[o], dx[o]);
 }
 // the right-hand side a factorisation is tried on: of magnitude one everywhere, no pattern
+// (the index hashed with the multipliers and shifts of the xxHash32 finaliser)
 __global__ void k_fd_probe(double2* f, size_t n) {
     for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
         unsigned h = (unsigned)o * 2654435761u;
@@ -935,7 +936,7 @@ struct orf_fdfd {
     int nx = 0, nz = 0, m = 0, nb = 0, C = 8;
     bool along_x = true;   // blocks are lines of constant x (m = nz)
     int S = 1, planned = 1;   // segments of the factors, and as chosen for the grid
-    double mnorm = 0.0;    // bound of the row sums of |M|
+    double mnorm = 0.0;    // scale of |M|: its largest row sum, the two couplings along an axis taken together
     Arena ar;
     double2 *diag = nullptr, *wc = nullptr, *eb = nullptr, *sx = nullptr, *sz = nullptr;
     double2 *inv = nullptr, *vin = nullptr, *vout = nullptr, *xrow = nullptr;
@@ -1123,8 +1124,8 @@ int orf_fdfd::factor(int nseg) {
         for (int q = 0; q < J; ++q) {
             // segment q before the separator (its last line eliminated last),
             // segment q + 1 after it (the last segment runs downwards)
-            const double2* first = q + 1 == S - 1 ? inv + (size_t)hs[S - 1].a * mm
-                                   : hs[q + 1].n == 1 ? inv + (size_t)hs[q + 1].a * mm : F + (size_t)q * mm;
+            // (a segment has four lines at least: F of every one with two separators)
+            const double2* first = q + 1 == S - 1 ? inv + (size_t)hs[S - 1].a * mm : F + (size_t)q * mm;
             si[q] = FdSepIn{sep[q], q > 0 ? 1 : 0, inv + (size_t)(sep[q] - 1) * mm, first,
                             q > 0 ? Lp(q, hs[q].n - 1) : nullptr};
         }
