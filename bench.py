@@ -335,6 +335,11 @@ def bench_pixel2d(args, rank, world, local, dist):
         if not coupler:
             tpc = ncu_traffic_per_cell_update()
             roof["traffic"] = tpc * roof["cell_updates_per_launch"] if tpc else None
+            if tpc:   # the DRAM bytes of the capture over this run's launch time
+                roof["traffic_frac"] = roof["traffic"] / (roof["avg_launch_ms"] / 1e3) / 1e9 / roof["peak"]
+        # T fused steps move the fields once: the bytes are those of a kernel
+        # that moves them every step, so frac is no bound and may pass one
+        roof["frac_note"] = "algorithmic bytes of one pass per time step; the launches fuse T steps per pass"
         roof["share_of_step_kernels"] = st["interior_ms"] / max(1e-9, st["interior_ms"] + st["frame_ms"])
         roof["frame_kernel_avg_launch_ms"] = st["frame_ms"] / max(1, st["frame_launches"])
         roof["frame_share_of_cell_updates"] = st["frame_cell_updates"] / max(

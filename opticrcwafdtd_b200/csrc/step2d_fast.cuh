@@ -583,9 +583,10 @@ k_step2d_fast(const FastTile2D* __restrict__ tiles, int ntiles, int launch_off, 
                     if (d.flags & 6) {      // DFT monitor samples of this step
                         // FP32 interior tiles: worked out anew in each step.  Hoisted
                         // out of the loop, the addresses of this path hold registers
-                        // that the 64 of a thread do not have: 35 spilled instead of
-                        // 10, and an interior launch of 4000 x 1500 TM takes 159 us
-                        // instead of 141 (FP64: 71 us against 74 on 1611 x 707)
+                        // that the 64 of a thread do not have: 25 words spilled
+                        // instead of 14 (TE 34 instead of 10), and an interior launch
+                        // of 4000 x 1500 TM (7 steps on average) takes 159 us instead
+                        // of 141 (FP64: 71 us against 74 on 1611 x 707)
                         int kq = kb, iq = i;
                         unsigned ownq = own;
                         if (!PML && sizeof(R) == 4) asm volatile("" : "+r"(kq), "+r"(iq), "+r"(ownq));
