@@ -41,6 +41,7 @@
 #include <math_constants.h>
 
 #include <complex>
+#include <limits>
 
 #include "runtime.cuh"
 
@@ -714,17 +715,10 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_red(FdfdDev P, FdRed D, const do
     cl.sync();   // no CTA leaves while another may still write its shared memory
 }
 
-// Power of two that brings the largest entry of a right-hand side to [1, 2):
-// its exponent (0 where there is none to take, an entry not finite or all zero).
-// big: the bits of the largest |re| or |im|.  A solve with it is the same to the
-// bit, and the squares in its residual neither vanish nor overflow.
-__device__ __forceinline__ int fd_exponent(const unsigned long long* big) {
-    const double v = big ? __longlong_as_double((long long)*big) : 0.0;
-    return v > 0.0 && v < CUDART_INF ? ilogb(v) : 0;
-}
 __device__ __forceinline__ double2 fd_scaled(double2 a, int e) {
     return e == 0 ? a : make_double2(scalbn(a.x, e), scalbn(a.y, e));
 }
+// bits of the largest |re| or |im| (infinity's where an entry is not finite)
 __global__ void k_fd_biggest(const double2* __restrict__ v, size_t n, unsigned long long* big) {
     double a = 0.0;
     bool nan = false;
@@ -741,16 +735,16 @@ __global__ void k_fd_biggest(const double2* __restrict__ v, size_t n, unsigned l
 
 // The caller's vector (i + nx k) and the block layout (b m + p), with the
 // scaling by s = s_x(i) s_z(k): f = -s J (mode 0) or g (mode 1); E = x or s x.
-// big: the largest entry of the caller's vector, to whose scale f is brought
-// (null: f is not scaled).
+// f is taken by 2^-ex and the result by 2^ex.  k_fd_in clears mx for the residual
+// that follows.
 struct FdMap {
     int nx, nz, along_x;
     const double2 *sx, *sz;
     __device__ size_t at(int i, int k) const { return along_x ? (size_t)i * nz + k : (size_t)k * nx + i; }
 };
 __global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __restrict__ f, int mode,
-                        const unsigned long long* big) {
-    const int ex = fd_exponent(big);
+                        int ex, unsigned long long* mx) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) mx[threadIdx.x] = 0;
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
          g += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
@@ -763,8 +757,7 @@ __global__ void k_fd_in(FdMap mp, const double2* __restrict__ v, double2* __rest
     }
 }
 __global__ void k_fd_out(FdMap mp, const double2* __restrict__ x, double2* __restrict__ v, int mode,
-                         const unsigned long long* big) {
-    const int ex = fd_exponent(big);
+                         int ex) {
     for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < (size_t)mp.nx * mp.nz;
          g += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(g % mp.nx), k = (int)(g / mp.nx);
@@ -802,13 +795,16 @@ __global__ void k_fd_residual(FdfdDev P, const double2* __restrict__ f, const do
         if ((threadIdx.x & 31) == 0) atomicMax(mx + q, (unsigned long long)__double_as_longlong(v[q]));
     }
 }
-__global__ void k_fd_add(double2* __restrict__ x, const double2* __restrict__ dx, size_t n) {
+// x += dx; clears mx for the residual that follows
+__global__ void k_fd_add(double2* __restrict__ x, const double2* __restrict__ dx, size_t n, unsigned long long* mx) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) mx[threadIdx.x] = 0;
     for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x)
         x[o] = cadd(x[o], dx[o]);
 }
 // the right-hand side a factorisation is tried on: of magnitude one everywhere, no pattern
 // (the index hashed with the multipliers and shifts of the xxHash32 finaliser)
-__global__ void k_fd_probe(double2* f, size_t n) {
+__global__ void k_fd_probe(double2* f, size_t n, unsigned long long* mx) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) mx[threadIdx.x] = 0;
     for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
         unsigned h = (unsigned)o * 2654435761u;
         h ^= h >> 15;
@@ -942,8 +938,9 @@ struct orf_fdfd {
     double2 *inv = nullptr, *vin = nullptr, *vout = nullptr, *xrow = nullptr;
     double2 *f = nullptr, *x = nullptr, *r = nullptr, *dx = nullptr, *Y = nullptr, *YT = nullptr, *V = nullptr,
             *Z = nullptr;
-    unsigned long long* mx = nullptr;   // largest |r|^2, |x|^2, |f|^2; largest entry of the caller's right-hand side
+    unsigned long long* mx = nullptr;   // largest |r|^2, |x|^2, |f|^2; the caller's largest entry (k_fd_biggest)
     double* h_mx = nullptr;             // the same on the host (pinned)
+    int scale = 0;                      // of f
     double eta = -1.0;                  // residual of the last solve (-1: none taken)
     bool singular = false;              // a zero or NaN pivot in the last factorisation
     FdSeg* segs = nullptr;
@@ -974,13 +971,19 @@ struct orf_fdfd {
         }
         return ORF_OK;
     }
-    // r = f - M x on the stream; its size reaches the host with it
+    // f of the caller's right-hand side (in vin), taken by 2^-scale
+    int rhs(int mode) {
+        k_fd_in<<<296, 256, 0, ctx->stream>>>(map(), vin, f, mode, scale, mx);
+        ORF_CUDA(cudaGetLastError());
+        return ORF_OK;
+    }
+    // r = f - M x on the stream; its size reaches the host with it (mx cleared by
+    // the kernel that formed f or x)
     int residual() {
         cudaStream_t st = ctx->stream;
-        ORF_CUDA(cudaMemsetAsync(mx, 0, 3 * sizeof *mx, st));
         k_fd_residual<<<296, 256, 0, st>>>(dev(), f, x, r, mx);
         ORF_CUDA(cudaGetLastError());
-        ORF_CUDA(cudaMemcpyAsync(h_mx, mx, 4 * sizeof *mx, cudaMemcpyDeviceToHost, st));
+        ORF_CUDA(cudaMemcpyAsync(h_mx, mx, 3 * sizeof *mx, cudaMemcpyDeviceToHost, st));
         return ORF_OK;
     }
     // its size against rounding, |r| / (|M| |x| + |f|) with the largest entries,
@@ -991,12 +994,13 @@ struct orf_fdfd {
     }
     int refine() {
         ORF_TRY(solve(r, dx));
-        k_fd_add<<<296, 256, 0, ctx->stream>>>(x, dx, N());
+        k_fd_add<<<296, 256, 0, ctx->stream>>>(x, dx, N(), mx);
         ORF_CUDA(cudaGetLastError());
         return ORF_OK;
     }
     template <class Out>
-    int settle(Out&& out);
+    int settle(int mode, Out&& out);
+    int scaled(int mode, bool* finite);
     int factor(int nseg);
     int refuse_singular() const {
         if (!singular) return ORF_OK;
@@ -1018,17 +1022,44 @@ constexpr double kEtaRefine = 1e-16, kEtaAccept = 1e-15, kEtaTrial = 1e-11;
 constexpr int kRefineSteps = 3;
 }  // namespace
 
+// The residual's squares vanish or overflow, or it is not a number: the right-hand
+// side brought to [1, 2) by a power of two, and solved again.  The result is the same to the bit as at an
+// ordinary magnitude.  finite: false where an entry is not, or all are zero (there
+// is nothing to refine).
+int orf_fdfd::scaled(int mode, bool* finite) {
+    cudaStream_t st = ctx->stream;
+    ORF_CUDA(cudaMemsetAsync(mx + 3, 0, sizeof *mx, st));
+    k_fd_biggest<<<296, 256, 0, st>>>(vin, N(), mx + 3);
+    ORF_CUDA(cudaGetLastError());
+    ORF_CUDA(cudaMemcpyAsync(h_mx + 3, mx + 3, sizeof *mx, cudaMemcpyDeviceToHost, st));
+    ORF_CUDA(cudaStreamSynchronize(st));
+    *finite = std::isfinite(h_mx[3]) && h_mx[3] > 0.0;
+    if (!*finite) return ORF_OK;
+    scale = std::ilogb(h_mx[3]);
+    ORF_TRY(rhs(mode));
+    ORF_TRY(solve(f, x));
+    ORF_TRY(residual());
+    ORF_CUDA(cudaStreamSynchronize(st));
+    return ORF_OK;
+}
+
 // From the first x of M x = f to the one handed over by out(), which waits for
 // the stream: refined as above, the result under way while the residual of the
-// step before it is taken (out() runs again in the rare case that more is to
-// do).  A right-hand side that is not finite (h_mx[3]: its largest entry) has no
-// residual.
+// step before it is taken (out() runs again in the rare case that more is to do).
 template <class Out>
-int orf_fdfd::settle(Out&& out) {
+int orf_fdfd::settle(int mode, Out&& out) {
     ORF_TRY(residual());
     ORF_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (!(h_mx[2] > 1e-200 && h_mx[2] < 1e200) || !std::isfinite(eta_now())) {
+        bool finite = false;
+        ORF_TRY(scaled(mode, &finite));
+        if (!finite) {
+            eta = h_mx[3] == 0.0 ? 0.0 : std::numeric_limits<double>::quiet_NaN();
+            return out();
+        }
+    }
     eta = eta_now();
-    if (!std::isfinite(h_mx[3]) || eta <= (S > 1 ? kEtaRefine : kEtaAccept)) return out();
+    if (eta <= (S > 1 ? kEtaRefine : kEtaAccept)) return out();
     for (int k = 0; k < kRefineSteps; ++k) {
         const double before = eta;
         ORF_TRY(refine());
@@ -1041,8 +1072,9 @@ int orf_fdfd::settle(Out&& out) {
     if (S == 1) return ORF_OK;
     ORF_TRY(factor(1));
     ORF_TRY(refuse_singular());
+    ORF_TRY(rhs(mode));
     ORF_TRY(solve(f, x));
-    return settle(out);
+    return settle(mode, out);
 }
 
 // Factor the operator as nseg segments.
@@ -1315,7 +1347,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         // a segment that is nearly singular by itself shows in a trial solve
         double trial = 0.0;
         if (!F->singular) {
-            k_fd_probe<<<296, 256, 0, st>>>(F->f, N);
+            k_fd_probe<<<296, 256, 0, st>>>(F->f, N, F->mx);
             ORF_CUDA(cudaGetLastError());
             ORF_TRY(F->solve(F->f, F->x));
             ORF_TRY(F->residual());
@@ -1351,23 +1383,16 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
     } rel{stage, st};
     ORF_TRY(copy_h2d_staged(F->vin, rhs, bytes, stage, st));
     add_h2d(F->ctx, (int64_t)bytes);
-    // (planned as one segment: no residual is taken, nothing to scale for)
-    const bool checked = F->planned > 1;
-    unsigned long long* big = checked ? F->mx + 3 : nullptr;
-    if (checked) {
-        ORF_CUDA(cudaMemsetAsync(big, 0, sizeof *big, st));
-        k_fd_biggest<<<296, 256, 0, st>>>(F->vin, F->N(), big);
-        ORF_CUDA(cudaGetLastError());
-    }
-    k_fd_in<<<296, 256, 0, st>>>(F->map(), F->vin, F->f, mode, big);
-    ORF_CUDA(cudaGetLastError());
+    F->scale = 0;
+    ORF_TRY(F->rhs(mode));
     auto result = [&]() -> int {   // of the solve so far, into the caller's array
-        k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, big);
+        k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, F->scale);
         ORF_CUDA(cudaGetLastError());
         return copy_d2h_staged(x, F->vout, bytes, stage, st);
     };
     ORF_TRY(F->solve(F->f, F->x));
-    ORF_TRY(checked ? F->settle(result) : result());
+    // (planned as one segment: no residual is taken)
+    ORF_TRY(F->planned > 1 ? F->settle(mode, result) : result());
     add_d2h(F->ctx, (int64_t)bytes);
     return ORF_OK;
 }

@@ -239,3 +239,22 @@ def test_fdfd_segments_near_resonance(detuning):
             assert rel(a(J), b(J)) <= TOL
             assert 0.0 <= o.info()["residual"] <= 1e-15
     o.close()
+
+
+def test_fdfd_source_that_has_no_residual():
+    """A source with a NaN or an infinity, and one of zeros, are solved as they
+    are: the factors stay, and the next solve is the first one's to the bit."""
+    x, z, eps, lam, J, g, npml = fdfd_cases.random_problem(120, 40, 4, True)
+    o = orf.fdfd2D(x, z, eps, lam, J, Npml=npml)
+    planned = o.info()["planned_segments"]
+    assert planned > 1
+    for bad in (np.nan, np.inf):
+        Jb = J.copy()
+        Jb[60, 20] = bad
+        assert not np.all(np.isfinite(o.solve(Jb)))
+        assert np.isnan(o.info()["residual"])
+    assert np.all(o.solve(0 * J) == 0) and np.all(o.adjoint(0 * g) == 0)
+    assert o.info()["residual"] == 0.0
+    assert np.array_equal(o.solve(J), o.E)
+    assert o.info()["segments"] == planned and 0.0 < o.info()["residual"] <= 1e-15
+    o.close()
