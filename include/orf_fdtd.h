@@ -208,9 +208,9 @@ ORF_API int32_t orf_ctx_get_stats(orf_ctx* ctx, orf_kernel_stats* st);
  * plane copies it still has in flight, and later launches of the run return
  * at once).  stall_plane >= 0 is a failure-detection test hook: in 3D jobs
  * created on this context afterwards, every tile loaded by TMA arms the ring
- * slot of its z-plane k0 + stall_plane (of its last one, where its segment is
- * shorter) without issuing the copies, so that wait runs out; -1 (the default)
- * turns it off.  Runs created before the call
+ * slot of its z-plane k0 + stall_plane (or that of the last plane of the run's
+ * shortest segment) without issuing the copies, so that wait runs out; -1 (the
+ * default) turns it off.  Runs created before the call
  * keep their launch arguments (CUDA graphs). */
 ORF_API int32_t orf_ctx_set_wait_injection(orf_ctx* ctx, int32_t stall_plane, int64_t wait_ns);
 ORF_API int32_t orf_ctx_reset_stats(orf_ctx* ctx);

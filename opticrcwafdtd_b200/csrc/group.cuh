@@ -245,17 +245,18 @@ struct Group3D : Group {
         nt = (int)tl.size();
         ntp = (int)tp.size();
         const bool f64 = sizeof(R) == 8;
+        const int shortest = shortest3d(tl, tp);
         wire_engine(f64, 1);
         if (nt && ntp) ORF_TRY(side.init());
-        eng.step = [this, f64](int off, int nsub, int par, int we, cudaStream_t s, KernelTimer* tm) -> cudaError_t {
+        eng.step = [this, f64, shortest](int off, int nsub, int par, int we, cudaStream_t s, KernelTimer* tm) -> cudaError_t {
             (void)nsub;
             cudaEvent_t a = nullptr;
             if (tm && tm->begin(s, &a) != ORF_OK) return cudaErrorUnknown;
             const bool overlap = !tm && side.ok() && nt && ntp;
             cudaError_t e = overlap ? side.fork(s) : cudaSuccess;
-            if (e == cudaSuccess) e = launch_step3d(f64, false, idxw, d_insts, d_tiles, nt, par, off, we, wait_ctl(ctx), s);
+            if (e == cudaSuccess) e = launch_step3d(f64, false, idxw, d_insts, d_tiles, nt, par, off, we, wait_ctl(ctx, shortest), s);
             if (e == cudaSuccess)
-                e = launch_step3d(f64, true, idxw, d_insts, d_tiles_pml, ntp, par, off, we, wait_ctl(ctx),
+                e = launch_step3d(f64, true, idxw, d_insts, d_tiles_pml, ntp, par, off, we, wait_ctl(ctx, shortest),
                                   overlap ? side.s2 : s);
             if (e == cudaSuccess && overlap) e = side.join(s);
             if (e != cudaSuccess) return e;

@@ -273,6 +273,13 @@ void cut3d(const Layout3D& a, SegLen3D len, int inst, std::vector<Tile3D>& tiles
             }
 }
 
+int shortest3d(const std::vector<Tile3D>& tiles, const std::vector<Tile3D>& tiles_pml) {
+    int n = kSeg3;
+    for (const auto* l : {&tiles, &tiles_pml})
+        for (const Tile3D& t : *l) n = std::min(n, t.k1 - t.k0);
+    return n;
+}
+
 template <class R>
 int Job3D<R>::create(const orf_sim3d* s) {
     ORF_TRY(validate3d(s, slab, false));   // every caller scanned the permittivity already
@@ -660,7 +667,8 @@ int Job3D<R>::create(const orf_sim3d* s) {
     for (const Tile3D& t : tiles) ncell_int += (int64_t)t.tw * t.th * (t.k1 - t.k0);
     for (const Tile3D& t : tiles_pml) ncell_pml += (int64_t)t.tw * t.th * (t.k1 - t.k0);
     if (!tiles.empty() && !tiles_pml.empty()) ORF_TRY(side.init());
-    eng.step = [this, ncell_int, ncell_pml](int off, int nsub, int par, int we, cudaStream_t stream,
+    const int shortest = shortest3d(tiles, tiles_pml);
+    eng.step = [this, ncell_int, ncell_pml, shortest](int off, int nsub, int par, int we, cudaStream_t stream,
                                             KernelTimer* tm) -> cudaError_t {
         (void)nsub;
         cudaEvent_t a = nullptr;
@@ -672,13 +680,13 @@ int Job3D<R>::create(const orf_sim3d* s) {
         cudaError_t e = overlap ? side.fork(stream) : cudaSuccess;
         if (e == cudaSuccess && !tiles.empty()) {
             if (tm && tm->begin(stream, &a) != ORF_OK) return cudaErrorUnknown;
-            e = launch_step3d(f64, false, idxw, d_inst, d_tiles, (int)tiles.size(), par, off, we, wait_ctl(ctx), stream);
+            e = launch_step3d(f64, false, idxw, d_inst, d_tiles, (int)tiles.size(), par, off, we, wait_ctl(ctx, shortest), stream);
             if (e == cudaSuccess && tm && tm->end(stream, 0, ncell_int, a) != ORF_OK) return cudaErrorUnknown;
         }
         if (e == cudaSuccess && !tiles_pml.empty()) {
             if (tm && tm->begin(stream, &a) != ORF_OK) return cudaErrorUnknown;
             e = launch_step3d(f64, true, idxw, d_inst, d_tiles_pml, (int)tiles_pml.size(), par, off, we,
-                              wait_ctl(ctx), overlap ? side.s2 : stream);
+                              wait_ctl(ctx, shortest), overlap ? side.s2 : stream);
             if (e == cudaSuccess && tm && tm->end(stream, 1, ncell_pml, a) != ORF_OK) return cudaErrorUnknown;
         }
         if (e == cudaSuccess && overlap) e = side.join(stream);

@@ -26,6 +26,8 @@ Layout3D layout3d(const orf_sim3d* s, bool zlo = true, bool zhi = true);
 SegLen3D seg_lengths(const std::vector<const Layout3D*>& runs, bool fp64, int sm_count);
 // append the run's interior and CPML tiles, as instance inst
 void cut3d(const Layout3D& lay, SegLen3D len, int inst, std::vector<Tile3D>& tiles, std::vector<Tile3D>& tiles_pml);
+// planes of the shortest segment
+int shortest3d(const std::vector<Tile3D>& tiles, const std::vector<Tile3D>& tiles_pml);
 
 template <class R>
 struct Job3D : orf_job {

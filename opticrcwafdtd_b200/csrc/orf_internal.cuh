@@ -226,8 +226,8 @@ constexpr int kSeg3 = 60;                  // z planes marched by one 3D CTA
 // the plane below the segment included) near a CPML slab.
 // Bounds of the 3D kernel's plane waits: wait_ns per plane (0: one second);
 // stall_plane >= 0 is the failure-detection test hook (the plane k0 +
-// stall_plane of every TMA tile, or its last one in a shorter segment, is armed
-// but never loaded, so its wait runs out), -1 in every production launch.
+// stall_plane of every TMA tile is armed but never loaded, so its wait runs
+// out), -1 in every production launch.
 struct WaitCtl {
     unsigned long long wait_ns;
     int stall_plane;

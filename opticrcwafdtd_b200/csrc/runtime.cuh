@@ -249,7 +249,10 @@ struct orf_ctx {
 };
 
 namespace orf {
-inline WaitCtl wait_ctl(const orf_ctx* c) { return WaitCtl{c->wait_ns, c->stall_plane}; }
+// shortest: planes of the launch's shortest segment, which every tile has
+inline WaitCtl wait_ctl(const orf_ctx* c, int shortest) {
+    return WaitCtl{c->wait_ns, std::min(c->stall_plane, shortest - 1)};
+}
 // host-to-device byte counter of a context, safe from several host threads
 void add_h2d(orf_ctx* c, int64_t bytes);
 void add_d2h(orf_ctx* c, int64_t bytes);

@@ -412,8 +412,7 @@ k_step3d(const Inst3D<R>* __restrict__ insts, const Tile3D* __restrict__ tiles, 
                 s_issued = p;
                 // failure-detection test hook (off unless set on the host):
                 // the slot is armed but its copies are never issued
-                // (a shorter segment's last plane)
-                if (wc.stall_plane >= 0 && p == k0 + min(wc.stall_plane, k1 - 1 - k0)) return;
+                if (wc.stall_plane >= 0 && p == k0 + wc.stall_plane) return;
                 for (int q = 0; q < 3; ++q) {
                     tma_load3(sEq(s2, q), tm + 128 * (3 * par + q), i0 - 4, j0 - 1, zc, &sbar[s2]);
                     tma_load3(sHq(s2, q), tm + 128 * (6 + 3 * par + q), i0 - 4, j0 - 1, zc, &sbar[s2]);

@@ -48,8 +48,8 @@ class Context:
         """Bounds of the 3D kernel's device-side plane waits (wait_ns per
         wait; 0 = one second) and the failure-detection test hook: with
         stall_plane >= 0, 3D jobs created afterwards on this context never
-        load that z-plane of their tiles (the last one of shorter segments), so
-        the wait runs out and the run ends with orf:deviceTimeout
+        load that z-plane of their tiles (at most the last of the shortest
+        segment), so the wait runs out and the run ends with orf:deviceTimeout
         (orf_ctx_set_wait_injection)."""
         _lib.check(self._lib.orf_ctx_set_wait_injection(self.handle, int(stall_plane), int(wait_ns)),
                    "orf_ctx_set_wait_injection")
