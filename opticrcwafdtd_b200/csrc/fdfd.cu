@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(NT, 1) k_fdfd_factor(FdfdDev P, const FdSeg* _
                         pr[l] = cfma(g, prw[l], base);
                     }
                     pr[aa] = g;
-                    if (me && !(dd > 0.0)) atomicExch(P.fault, 1);   // a zero or NaN pivot
+                    // a zero or NaN pivot (as bits: a quiet NaN's key, no further FP64 comparison)
+                    if (me && (dd == 0.0 || bk >= 0x7ff80000)) atomicExch(P.fault, 1);
                 }
                 if (t >= r0 && t < r0 + nr) {
                     s_kown[t - r0] = (signed char)myk;
@@ -945,11 +946,13 @@ struct orf_fdfd {
     bool singular = false;              // a zero or NaN pivot in the last factorisation
     FdSeg* segs = nullptr;
     int *line = nullptr, *fault = nullptr;
+    cudaEvent_t copied = nullptr;       // the result has reached the staging buffer
     ~orf_fdfd() {
         if (ar.base) {
             cudaStreamSynchronize(ctx->stream);
             ar.release();
         }
+        if (copied) cudaEventDestroy(copied);
         host_mapped_free(h_mx);
         if (ctx) ctx_release(ctx);
     }
@@ -1043,9 +1046,10 @@ int orf_fdfd::scaled(int mode, bool* finite) {
     return ORF_OK;
 }
 
-// From the first x of M x = f to the one handed over by out(), which waits for
-// the stream: refined as above, the result under way while the residual of the
-// step before it is taken (out() runs again in the rare case that more is to do).
+// From the first x of M x = f to the one handed over by out(beside), which enqueues
+// the copy, then beside, and waits for the copy: refined as above, the residual of
+// the refined x taken while the host moves the result (out runs again in the rare
+// case that more is to do).
 template <class Out>
 int orf_fdfd::settle(int mode, Out&& out) {
     ORF_TRY(residual());
@@ -1055,16 +1059,16 @@ int orf_fdfd::settle(int mode, Out&& out) {
         ORF_TRY(scaled(mode, &finite));
         if (!finite) {
             eta = h_mx[3] == 0.0 ? 0.0 : std::numeric_limits<double>::quiet_NaN();
-            return out();
+            return out([]() -> int { return ORF_OK; });
         }
     }
     eta = eta_now();
-    if (eta <= (S > 1 ? kEtaRefine : kEtaAccept)) return out();
+    if (eta <= (S > 1 ? kEtaRefine : kEtaAccept)) return out([]() -> int { return ORF_OK; });
     for (int k = 0; k < kRefineSteps; ++k) {
         const double before = eta;
         ORF_TRY(refine());
-        ORF_TRY(residual());
-        ORF_TRY(out());
+        ORF_TRY(out([this] { return residual(); }));
+        ORF_CUDA(cudaStreamSynchronize(ctx->stream));
         eta = eta_now();
         if (eta <= kEtaAccept) return ORF_OK;
         if (!(eta < before)) break;   // it falls no more (or is not a number)
@@ -1321,6 +1325,7 @@ extern "C" int32_t orf_fdfd2d_factor(orf_ctx* ctx, const orf_fdfd2d* pr, orf_fdf
         void *h = nullptr, *d = nullptr;
         ORF_TRY(host_mapped_alloc(4 * sizeof(double), &h, &d));
         F->h_mx = static_cast<double*>(h);
+        ORF_CUDA(cudaEventCreateWithFlags(&F->copied, cudaEventDisableTiming));
     }
     int rc = carve();
     if (rc == ORF_ENOMEM_DEVICE && S > 1) {   // one segment needs no memory for separators
@@ -1385,14 +1390,23 @@ extern "C" int32_t orf_fdfd2d_solve(orf_fdfd* F, const double* rhs, double* x, i
     add_h2d(F->ctx, (int64_t)bytes);
     F->scale = 0;
     ORF_TRY(F->rhs(mode));
-    auto result = [&]() -> int {   // of the solve so far, into the caller's array
+    auto result = [&](auto&& beside) -> int {   // of the solve so far, into the caller's array
         k_fd_out<<<296, 256, 0, st>>>(F->map(), F->x, F->vout, mode, F->scale);
         ORF_CUDA(cudaGetLastError());
-        return copy_d2h_staged(x, F->vout, bytes, stage, st);
+        const char* src = reinterpret_cast<const char*>(F->vout);
+        for (size_t off = 0; off < bytes; off += kStageBytes) {
+            const size_t n = std::min(kStageBytes, bytes - off);
+            ORF_CUDA(cudaMemcpyAsync(stage, src + off, n, cudaMemcpyDeviceToHost, st));
+            ORF_CUDA(cudaEventRecord(F->copied, st));
+            if (off + n == bytes) ORF_TRY(beside());
+            ORF_CUDA(cudaEventSynchronize(F->copied));
+            std::memcpy(reinterpret_cast<char*>(x) + off, stage, n);
+        }
+        return ORF_OK;
     };
     ORF_TRY(F->solve(F->f, F->x));
     // (planned as one segment: no residual is taken)
-    ORF_TRY(F->planned > 1 ? F->settle(mode, result) : result());
+    ORF_TRY(F->planned > 1 ? F->settle(mode, result) : result([]() -> int { return ORF_OK; }));
     add_d2h(F->ctx, (int64_t)bytes);
     return ORF_OK;
 }
